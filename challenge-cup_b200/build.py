@@ -16,7 +16,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "ertm_b200" / "libertm_b200.so"
-SOURCES = [CSRC / "ertm_b200.cu"]
+SOURCES = [CSRC / "ertm_b200.cu", CSRC / "wave.cu"]
 DEPS = sorted(CSRC.glob("*.cu*")) + [HERE.parent / "include" / "ertm_b200.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -37,18 +37,27 @@ def up_to_date() -> bool:
 def build(force: bool = False, ptxas_verbose: bool = False) -> Path:
     if not force and up_to_date():
         return OUT
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
-           "-Xcompiler", "-fPIC,-O3", "-shared", "-o", str(OUT), *map(str, SOURCES), "-lcufft"]
+    flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-O3"]
     if ptxas_verbose:
-        cmd.insert(1, "-Xptxas=-v")
+        flags.append("-Xptxas=-v")
+    objects = [OUT.parent / f"{src.stem}.o" for src in SOURCES]
+    # the translation units compile side by side
+    procs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(obj), str(src)], stdout=subprocess.PIPE,
+                              stderr=subprocess.STDOUT, text=True) for src, obj in zip(SOURCES, objects)]
+    logs = [p.communicate()[0] for p in procs]
     tmp = OUT.with_suffix(".so.tmp")
-    cmd[cmd.index(str(OUT))] = str(tmp)
-    res = subprocess.run(cmd, capture_output=True, text=True)
+    link = [nvcc(), *ARCH, "-shared", "-o", str(tmp), *map(str, objects), "-lcufft"]
+    for p, log in zip(procs, logs):
+        if p.returncode != 0 or ptxas_verbose:
+            sys.stderr.write(log)
+    if any(p.returncode != 0 for p in procs):
+        raise RuntimeError("nvcc failed")
+    res = subprocess.run(link, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError(f"nvcc failed with exit code {res.returncode}")
-    if ptxas_verbose:
-        sys.stderr.write(res.stderr)
+        raise RuntimeError(f"nvcc (link) failed with exit code {res.returncode}")
+    for obj in objects:
+        obj.unlink()
     os.replace(tmp, OUT)
     return OUT
 

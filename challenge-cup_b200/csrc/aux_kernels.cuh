@@ -145,6 +145,30 @@ __global__ void k_sample(const DevProp* props, int pi, SampleSet S, int64_t row_
   sp.out[row_offset + r] = v;
 }
 
+// Receiver values from the corner cells of every step (k_sample's sum, term
+// for term): row k of `buf` holds (component, receiver, corner).
+__global__ void k_sample_corners(const float* __restrict__ buf, int64_t stride, SampleSet S, int n_steps,
+                                 int64_t row0) {
+  const int comp = blockIdx.z;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const SamplePlanDev& sp = S.plan[comp];
+  if (r >= sp.n) return;
+  const bool live = sp.kind != SAMPLE_ZERO && sp.valid[r];
+  const double w0 = sp.w[4 * r], w1 = sp.w[4 * r + 1], w2 = sp.w[4 * r + 2], w3 = sp.w[4 * r + 3];
+  for (int k = blockIdx.y; k < n_steps; k += gridDim.y) {
+    float v = 0.f;
+    if (live) {
+      const float4 q = ldg4(buf + (int64_t)k * stride + 4 * ((int64_t)comp * sp.n + r));
+      double acc = dmul(dmul((double)q.x, w0), w2);
+      acc = dadd(acc, dmul(dmul((double)q.y, w0), w3));
+      acc = dadd(acc, dmul(dmul((double)q.z, w1), w2));
+      acc = dadd(acc, dmul(dmul((double)q.w, w1), w3));
+      v = __double2float_rn(acc);
+    }
+    sp.out[(row0 + k) * sp.n + r] = v;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // time-reversed injection with np.add.at semantics (propagation.py:331-369,
 // 472-494, 916-942): every contribution is added in float64 and rounded to
@@ -285,12 +309,6 @@ __global__ void k_kahan_to_f64(const float* s, const float* c, double* out, int6
 // ---------------------------------------------------------------------------
 // viscoacoustic compensation safety net (propagation.py:726-749)
 // ---------------------------------------------------------------------------
-struct StabState {
-  double ref_amp;   // reference amplitude: running max|p| over steps < 30
-  int32_t clipped;  // amplitude-cap events
-  int32_t pad_;
-};
-
 __global__ void k_stab_reference(const DevProp* props, int pi, StabState* st) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const double peak = (double)*props[pi].peak;

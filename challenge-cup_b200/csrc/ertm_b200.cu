@@ -28,6 +28,7 @@
 #include "line_fft.cuh"
 #include "line_fft_plan.h"
 #include "step_kernels.cuh"
+#include "wave_kernel.cuh"
 
 using namespace ertm;
 
@@ -410,6 +411,8 @@ struct SamplePlanHost {
   int kind = SAMPLE_FIELD, slot = 0;
   DevBuf cell, valid, w;
   int n = 0;
+  std::vector<int32_t> h_cell;   // host copies (multi-step launches group them by CTA)
+  std::vector<uint8_t> h_valid;
 };
 
 struct InjectTarget {
@@ -418,9 +421,17 @@ struct InjectTarget {
   int scaled;        // 0: (v·w_z)·w_x; 1: v·((w_z·w_x)·1); 2: v·((w_z·w_x)·1/|K_R|)
 };
 
+// The cells of an injection plan grouped by the CTAs of a multi-step launch.
+struct WaveInjectHost {
+  DevBuf cta, slot, ij, start, src, wa, wb;
+};
+
 struct InjectPlanHost {
   DevBuf cell_field, cell_index, start, src, wa, wb;
   int n_cells = 0;
+  std::vector<int32_t> h_field, h_index, h_start, h_src;   // host copies
+  std::vector<double> h_wa, h_wb;
+  std::map<std::pair<int, int>, WaveInjectHost> wave;      // by (px, pz)
   InjectPlanDev dev() const {
     InjectPlanDev d{};
     d.n_cells = n_cells;
@@ -524,6 +535,8 @@ SamplePlanHost& sample_plan(Prop& P, int comp) {
     w[4 * r + 2] = 1 - tx;
     w[4 * r + 3] = tx;
   }
+  sp->h_cell = cell;
+  sp->h_valid = valid;
   sp->cell = DevBuf(n * sizeof(int32_t), P.st);
   sp->valid = DevBuf(n, P.st);
   sp->w = DevBuf(w.size() * sizeof(double), P.st);
@@ -648,6 +661,12 @@ InjectPlanHost& inject_plan(Prop& P, const std::vector<int>& comps, int64_t nt) 
   put(ip->wa, wa.data(), wa.size() * 8);
   put(ip->wb, wb.data(), wb.size() * 8);
   CK(cudaStreamSynchronize(P.st));
+  ip->h_field = std::move(cf);
+  ip->h_index = std::move(cidx);
+  ip->h_start = std::move(start);
+  ip->h_src = std::move(src);
+  ip->h_wa = std::move(wa);
+  ip->h_wb = std::move(wb);
   auto& ref = *ip;
   P.injects[key] = std::move(ip);
   return ref;
@@ -1606,9 +1625,501 @@ uint32_t read_status(const Prop& P, cudaStream_t st) {
 // The error of a run whose propagators flagged non-finite values.
 void require_finite(const ShotRun& R, cudaStream_t st, const std::string& what) {
   const uint32_t f = read_status(*R.F, st), b = read_status(*R.B, st);
+  if ((f | b) & STATUS_STALLED) throw Error(ERTM_ERR_STATE, what + ": a wait between the CTAs of a launch ran out");
   if ((f | b) & STATUS_NONFINITE)
     throw Error(ERTM_ERR_NONFINITE, what + ": the " + std::string(f ? "source (forward/replay)" : "backward") +
                                         " wavefield became non-finite (NaN or infinity)");
+}
+
+// --------------------------------------------------------------------------
+// Multi-step launches (wave_kernel.cuh)
+// --------------------------------------------------------------------------
+// 0: where they are expected to be faster; 1: never; 2: wherever they fit.
+std::atomic<int> g_wave{0};
+constexpr int kWaveSmemMax = 227 * 1024 - 2048;   // dynamic shared memory (the static part left out)
+constexpr int kWaveMaxSteps = 1024;               // steps per launch: keeps a launch to a few ms
+
+int sm_count() {
+  static std::mutex mu;
+  static std::map<int, int> per_device;
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  int& n = per_device[dev];
+  if (n == 0) CK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  return n;
+}
+
+// How a propagator is split over at most `ncta` CTAs.
+struct WavePlan {
+  int px = 0, pz = 0, cells = 1;   // cells: per thread and pass
+  bool res = false;
+  int pad = 8;        // halo-field row padding (wave_layout)
+  int smem = 0;       // bytes
+  int64_t half = 0;   // exchange units per CTA and phase
+  bool ok() const { return px > 0; }
+  int ctas() const { return px * pz; }
+};
+
+// Largest shared-memory need of a split, in bytes.
+int wave_smem(const DevProp& h, const WavePlan& p, int n_epi) {
+  const int ng = (h.nxp + 3) / 4;
+  int most = 0;
+  for (int c = 0; c < p.px * p.pz; ++c) {
+    const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c);
+    int f, nsx, nsz;
+    wave_strip(4 * t.g0, std::min(4 * (t.g0 + t.gw), h.nxp), h.nxp, h.npx_l, h.npx_r, f, nsx);
+    wave_strip(t.i0, t.i0 + t.th, h.nzp, h.npz_t, h.npz_b, f, nsz);
+    const WaveLayout y = wave_layout(h.engine == ENGINE_ELASTIC, h.engine == ENGINE_VISCO, h.L, p.res, p.pad, t.th, t.gw, nsx, nsz, n_epi);
+    most = std::max(most, y.total * 4);
+  }
+  return most;
+}
+
+bool wave_supported(const DevProp& h) {
+  return h.M == 4 && h.fast_x == 1 && h.fast_z == 1 && h.nzp >= 8 && h.nxp >= 8 && h.nzp < 32768 && h.nxp < 32768 &&
+         (h.engine != ENGINE_VISCO || h.L <= kRelaxUnroll);
+}
+
+WavePlan wave_plan(const DevProp& h, int ncta, int n_epi) {
+  WavePlan best;
+  if (!wave_supported(h)) return best;
+  const int ng = (h.nxp + 3) / 4;
+  double cost = 0.0;
+  for (int px = 1; px <= std::min(ncta, ng); ++px) {
+    const int pz = std::min(ncta / px, h.nzp / WAVE_HALO);
+    if (pz < 1) continue;
+    const int th = (h.nzp + pz - 1) / pz, gw = (ng + px - 1) / px;
+    const double c = (double)(th + 2 * WAVE_HALO) * (4 * gw + 2 * WAVE_HALO);
+    if (best.px == 0 || c < cost) {
+      best.px = px;
+      best.pz = pz;
+      cost = c;
+    }
+  }
+  if (!best.ok()) return best;
+  const int th = (h.nzp + best.pz - 1) / best.pz, gw = (ng + best.px - 1) / best.px;
+  const int nx = h.engine == ENGINE_ELASTIC ? 2 : 1;
+  best.half = (int64_t)2 * nx * th + (int64_t)2 * nx * 4 * gw;
+  best.cells = th * 4 * gw <= WAVE_NT ? 1 : 2;
+  for (int k = 0; k < 4; ++k) {
+    best.res = k < 2;
+    best.pad = (k & 1) == 0 ? 32 : 8;
+    best.smem = wave_smem(h, best, n_epi);
+    if (best.smem <= kWaveSmemMax) return best;
+  }
+  best.px = 0;
+  return best;
+}
+
+// Exchange buffers of one driver call.  Epochs only grow, so words of earlier
+// launches never match; new memory is cleared (epoch 0 is never used).
+struct WaveRunner {
+  cudaStream_t st = nullptr;
+  DevBuf xbuf, peaks;
+  uint32_t epoch = 0;
+  WaveSet S{};
+  int grid = 0, smem = 0, engine = 0, cells = 1;
+  bool res = true;            // the works of a launch share engine, cells and res
+  double bytes = 0.0;
+  explicit WaveRunner(cudaStream_t s) : st(s) {}
+  void begin() {
+    S = WaveSet{};
+    grid = smem = 0;
+    bytes = 0.0;
+  }
+  // Add a work of `p.ctas()` CTAs; the caller fills in the rest.
+  WaveWork& add(const Prop& P, const WavePlan& p, int n_steps) {
+    WaveWork& w = S.w[S.n++];
+    engine = P.h.engine;
+    cells = p.cells;
+    res = p.res;
+    w.prop = P.dp();
+    w.cta0 = grid;
+    w.px = p.px;
+    w.pz = p.pz;
+    w.pad = p.pad;
+    w.n_steps = n_steps;
+    w.sign = 1;
+    grid += p.ctas();
+    smem = std::max(smem, p.smem);
+    S.half = std::max(S.half, p.half);
+    return w;
+  }
+  void launch() {
+    if (S.n == 0) return;
+    const size_t need = (size_t)grid * 2 * S.half * 32;
+    int most = 0;
+    for (int k = 0; k < S.n; ++k) most = std::max(most, S.w[k].n_steps);
+    if (xbuf.bytes < need || epoch > 0xf0000000u) {
+      if (xbuf.bytes < need) xbuf = DevBuf(need, st);
+      if (!peaks.p) peaks = DevBuf((size_t)2 * sm_count() * 8, st);
+      CK(cudaMemsetAsync(xbuf.p, 0, xbuf.bytes, st));
+      CK(cudaMemsetAsync(peaks.p, 0, peaks.bytes, st));
+      epoch = 0;
+    }
+    S.xbuf = xbuf.as<uint64_t>();
+    S.plane = (int64_t)grid * 2 * S.half * 2;
+    S.peaks = peaks.as<uint64_t>();
+    for (int k = 0; k < S.n; ++k) S.w[k].epoch = epoch;
+    epoch += 2 * (uint32_t)most + 2;
+    cudaEvent_t e0 = nullptr;
+    const bool timed = g_prof.begin(st, e0);
+    CK(wave_launch(engine, cells, res, S, grid, smem, kWaveSmemMax, st));
+    ++g_launches;
+    if (timed) g_prof.end(st, e0, bytes);
+  }
+};
+
+// CTA of each padded cell's row and column group.
+struct WaveOwner {
+  std::vector<int> tr, tc;
+  int px;
+  WaveOwner(const DevProp& h, const WavePlan& p) : tr(h.nzp), tc((h.nxp + 3) / 4), px(p.px) {
+    const int ng = (int)tc.size();
+    for (int c = 0; c < p.pz; ++c) {
+      const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c * p.px);
+      for (int i = 0; i < t.th; ++i) tr[t.i0 + i] = c;
+    }
+    for (int c = 0; c < p.px; ++c) {
+      const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c);
+      for (int g = 0; g < t.gw; ++g) tc[t.g0 + g] = c;
+    }
+  }
+  int of(int i, int j) const { return tr[i] * px + tc[j / 4]; }
+};
+
+DevBuf wave_upload(const void* data, size_t bytes, cudaStream_t st) {
+  DevBuf b(std::max<size_t>(bytes, 16), st);
+  upload(b.p, data, bytes, st);
+  return b;
+}
+
+const WaveInjectHost& wave_inject(const Prop& P, InjectPlanHost& plan, const WavePlan& p) {
+  auto it = plan.wave.find({p.px, p.pz});
+  if (it != plan.wave.end()) return it->second;
+  const WaveOwner own(P.h, p);
+  const int n = plan.n_cells, nc = p.ctas();
+  std::vector<int> cta(n);
+  std::vector<int32_t> first(nc + 1, 0);
+  for (int k = 0; k < n; ++k) {
+    cta[k] = own.of(plan.h_index[k] / P.h.ld, plan.h_index[k] % P.h.ld);
+    ++first[cta[k] + 1];
+  }
+  for (int c = 0; c < nc; ++c) first[c + 1] += first[c];
+  std::vector<int32_t> pos(first.begin(), first.end() - 1), order(n);
+  for (int k = 0; k < n; ++k) order[pos[cta[k]]++] = k;
+  std::vector<int32_t> slot(n), ij(n), start{0}, src;
+  std::vector<double> wa, wb;
+  for (int q = 0; q < n; ++q) {
+    const int k = order[q];
+    slot[q] = plan.h_field[k];
+    ij[q] = (plan.h_index[k] / P.h.ld) << 16 | (plan.h_index[k] % P.h.ld);
+    for (int c = plan.h_start[k]; c < plan.h_start[k + 1]; ++c) {
+      src.push_back(plan.h_src[c]);
+      wa.push_back(plan.h_wa[c]);
+      wb.push_back(plan.h_wb[c]);
+    }
+    start.push_back((int32_t)src.size());
+  }
+  WaveInjectHost w;
+  w.cta = wave_upload(first.data(), first.size() * 4, P.st);
+  w.slot = wave_upload(slot.data(), slot.size() * 4, P.st);
+  w.ij = wave_upload(ij.data(), ij.size() * 4, P.st);
+  w.start = wave_upload(start.data(), start.size() * 4, P.st);
+  w.src = wave_upload(src.data(), src.size() * 4, P.st);
+  w.wa = wave_upload(wa.data(), wa.size() * 8, P.st);
+  w.wb = wave_upload(wb.data(), wb.size() * 8, P.st);
+  CK(cudaStreamSynchronize(P.st));   // host vectors go out of scope
+  return plan.wave.emplace(std::make_pair(p.px, p.pz), std::move(w)).first->second;
+}
+
+// Receiver sampling of a set of components: corner cells grouped by CTA.
+struct WaveSampleHost {
+  DevBuf cta, slot, ij, out;
+};
+
+WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& comps, const WavePlan& p) {
+  const WaveOwner own(P.h, p);
+  struct Entry { int cta, slot, ij, out; };
+  std::vector<Entry> all;
+  const int ld = P.h.ld;
+  for (size_t c = 0; c < comps.size(); ++c) {
+    const SamplePlanHost& sp = *comps[c];
+    if (sp.kind == SAMPLE_ZERO) continue;
+    for (int r = 0; r < sp.n; ++r) {
+      if (!sp.h_valid[r]) continue;
+      for (int corner = 0; corner < 4; ++corner) {
+        const int i = sp.h_cell[r] / ld + (corner >> 1), j = sp.h_cell[r] % ld + (corner & 1);
+        all.push_back({own.of(i, j), sp.kind == SAMPLE_PRESSURE ? -1 : sp.slot, i << 16 | j,
+                       4 * ((int)c * sp.n + r) + corner});
+      }
+    }
+  }
+  const int nc = p.ctas();
+  std::vector<int32_t> first(nc + 1, 0), slot(all.size()), ij(all.size()), out(all.size());
+  for (const Entry& e : all) ++first[e.cta + 1];
+  for (int c = 0; c < nc; ++c) first[c + 1] += first[c];
+  std::vector<int32_t> pos(first.begin(), first.end() - 1);
+  for (const Entry& e : all) {
+    const int q = pos[e.cta]++;
+    slot[q] = e.slot;
+    ij[q] = e.ij;
+    out[q] = e.out;
+  }
+  WaveSampleHost w;
+  w.cta = wave_upload(first.data(), first.size() * 4, P.st);
+  w.slot = wave_upload(slot.data(), slot.size() * 4, P.st);
+  w.ij = wave_upload(ij.data(), ij.size() * 4, P.st);
+  w.out = wave_upload(out.data(), out.size() * 4, P.st);
+  CK(cudaStreamSynchronize(P.st));   // host vectors go out of scope
+  return w;
+}
+
+// Grids the multi-step launches are used for: whatever fits with the
+// coefficients resident.
+bool wave_wanted(const WavePlan& p) {
+  const int mode = g_wave.load();
+  return p.ok() && mode != 1 && (mode == 2 || p.res);
+}
+
+// Forward modelling through multi-step launches; false when the propagator
+// does not qualify.
+bool forward_wave(Prop& P, int nt, const float* dwave, const SampleSet& S, const std::vector<SamplePlanHost*>& comps) {
+  const bool comp = P.h.engine == ENGINE_VISCO && P.cfg.compensation;
+  if (nt < 2 || comp) return false;
+  const WavePlan p = wave_plan(P.h, sm_count(), 0);
+  if (!wave_wanted(p)) return false;
+  const int n = S.count ? S.plan[0].n : 0;
+  const int64_t stride = 4 * (int64_t)S.count * n;
+  WaveSampleHost sh;
+  if (stride) sh = wave_sample(P, comps, p);
+  // corner values of one launch: at most 32 MB
+  const int chunk = stride ? (int)std::max<int64_t>(16, std::min<int64_t>(kWaveMaxSteps, (int64_t(8) << 20) / stride))
+                           : kWaveMaxSteps;
+  DevBuf buf(stride ? (size_t)std::min(chunk, nt) * stride * 4 : 0, P.st);
+  WaveRunner run(P.st);
+  for (int t = 0; t < nt; t += chunk) {
+    const int m = std::min(chunk, nt - t);
+    run.begin();
+    WaveWork& w = run.add(P, p, m);
+    w.t0 = t;
+    w.wavelet = dwave;
+    if (stride) {
+      w.smp.cta = sh.cta.as<int32_t>();
+      w.smp.slot = sh.slot.as<int32_t>();
+      w.smp.ij = sh.ij.as<int32_t>();
+      w.smp.out = sh.out.as<int32_t>();
+      w.smp.buf = buf.as<float>();
+      w.smp.stride = stride;
+    }
+    run.bytes = m * step_bytes(P);
+    run.launch();
+    P.step_index += m;
+    if (stride) {
+      k_sample_corners<<<dim3((n + 127) / 128, (unsigned)std::min(m, 1024), S.count), 128, 0, P.st>>>(
+          buf.as<float>(), stride, S, m, t);
+      ++g_launches;
+      CK(cudaGetLastError());
+    }
+  }
+  return true;
+}
+
+// One shot through multi-step launches: the forward pass with checkpoints
+// written by the launches themselves, then, block by block, the replay of
+// block b − 1 beside the backward pass over block b (two works of one
+// launch, two replay buffers).  False when the shot does not qualify.
+struct WaveShot {
+  WavePlan whole, alone;   // the forward pass; a replay on every SM
+  WavePlan f, b;           // replay and backward, side by side where both fit
+};
+
+bool wave_shot(const ShotRun& R, WaveShot& W) {
+  const Prop& F = *R.F;
+  const Prop& B = *R.B;
+  if (R.fwd_unfused) return false;
+  if (F.h.engine == ENGINE_VISCO && F.cfg.compensation) return false;
+  const int n = sm_count();
+  const int nf = 1 + (F.h.engine == ENGINE_ELASTIC && R.need_src[1] ? 1 : 0);
+  const int nb = 1 + (F.h.engine == ENGINE_ELASTIC && R.need_rcv_s ? 1 : 0);
+  W.whole = wave_plan(F.h, n, 0);
+  if (!wave_wanted(W.whole)) return false;
+  // side by side on half the SMs each; one after the other on all of them
+  // when half the SMs cannot hold a propagator's resident arrays
+  W.alone = wave_plan(F.h, n, nf);
+  W.f = wave_plan(F.h, n / 2, nf);
+  W.b = wave_plan(B.h, n / 2, nb);
+  if (!W.f.ok() || !W.b.ok() || W.f.res != W.b.res || !W.f.res || W.f.cells != W.b.cells) {
+    W.f = W.alone;
+    W.b = wave_plan(B.h, n, nb);
+  }
+  return wave_wanted(W.alone) && wave_wanted(W.f) && wave_wanted(W.b);
+}
+
+bool wave_together(const WaveShot& W) { return W.f.ctas() + W.b.ctas() <= sm_count(); }
+
+void wave_set_inject(WaveWork& w, ShotRun& R, const WavePlan& p) {
+  if (!R.plan) return;
+  const WaveInjectHost& h = wave_inject(*R.B, *R.plan, p);
+  w.inj.cta = h.cta.as<int32_t>();
+  w.inj.slot = h.slot.as<int32_t>();
+  w.inj.ij = h.ij.as<int32_t>();
+  w.inj.start = h.start.as<int32_t>();
+  w.inj.src = h.src.as<int32_t>();
+  w.inj.wa = h.wa.as<double>();
+  w.inj.wb = h.wb.as<double>();
+  w.inj.record = R.rec.as<float>();
+  w.inj.nrec = R.nrec;
+}
+
+// n replay (or excitation-map) steps of block b from time t.
+void wave_add_replay(WaveRunner& run, ShotRun& R, const WavePlan& p, int b, int t, int n) {
+  WaveWork& w = run.add(*R.F, p, n);
+  w.t0 = t;
+  w.wavelet = R.wave.as<float>();
+  if (t == R.s_of(b)) {
+    w.load = R.ck.as<float>() + (size_t)b * R.F->state_floats;
+    R.F->step_index = R.ck_step[b];
+  }
+  w.epi = replay_epilogue(R, b, R.s_of(b));
+  w.slot_t = R.s_of(b);
+  w.slot_floats = (int64_t)R.n_src * (int64_t)R.npix;
+  R.F->step_index += n;
+  run.bytes += n * (step_bytes(*R.F) + epilogue_bytes(w.epi, R.npix));
+}
+
+// Backward steps of block b from time t down, at most `most`, up to and
+// including the next low-pass step; `lowpass` is its cutoff (0: none).
+int wave_add_backward(WaveRunner& run, ShotRun& R, const WavePlan& p, int b, int t, int most, double& lowpass) {
+  Prop& B = *R.B;
+  const bool comp = B.h.engine == ENGINE_VISCO && B.cfg.compensation;
+  const int every = B.cfg.lowpass_interval;
+  int n = most;
+  lowpass = 0.0;
+  if (comp && every > 1)
+    for (int k = 0; k < n; ++k) {
+      const int64_t s = B.step_index + k;
+      if (s >= 30 && s % every == 0) {
+        n = k + 1;
+        lowpass = std::max(0.9 - 0.4 * std::min((double)s * B.cfg.dt / 1.0, 1.0), 0.35);
+      }
+    }
+  WaveWork& w = run.add(B, p, n);
+  w.t0 = t;
+  w.sign = -1;
+  w.flags = (comp ? WAVE_STAB : 0) | (lowpass > 0.0 ? WAVE_SKIP_LAST : 0);
+  w.cap = B.cfg.amplitude_cap;
+  w.stab = B.stab.as<StabState>();
+  w.step_index = B.step_index;
+  const int s0 = R.excitation ? 0 : R.s_of(b);
+  w.epi = backward_epilogue(R, b, s0);
+  // the kernel decides per step what backward_epilogue decides per time
+  w.epi.kind = R.excitation ? EPI_EXC_IMAGE : EPI_IMAGE;
+  w.epi.cross = 1;
+  w.start_step = R.cfg.start_step;
+  w.slot_t = s0;
+  w.slot_floats = (int64_t)R.n_src * (int64_t)R.npix;
+  wave_set_inject(w, R, p);
+  B.step_index += n;
+  run.bytes += n * (step_bytes(B) + epilogue_bytes(w.epi, R.npix));
+  return n;
+}
+
+// After a launch whose backward work ended on a low-pass step: the low-pass,
+// then that step's imaging.
+void wave_finish_lowpass(ShotRun& R, int b, int t, double lowpass, cudaStream_t st) {
+  ++R.B->lowpass_steps;
+  lowpass_props({{R.B, lowpass}}, st);
+  const Epilogue e = backward_epilogue(R, R.excitation ? 0 : b, t);
+  if (e.kind != EPI_NONE) launch_epilogue(*R.B, e);
+}
+
+void wave_forward(WaveRunner& run, ShotRun& R, const WavePlan& p) {
+  Prop& F = *R.F;
+  for (int t = 0; t < R.nt; t += kWaveMaxSteps) {
+    const int m = std::min(kWaveMaxSteps, R.nt - t);
+    run.begin();
+    WaveWork& w = run.add(F, p, m);
+    w.t0 = t;
+    w.wavelet = R.wave.as<float>();
+    w.ck = R.ck.as<float>();
+    w.ck_every = R.iv;
+    w.ck_floats = (int64_t)F.state_floats;
+    for (int b = (t + R.iv - 1) / R.iv; b < R.n_states && R.s_of(b) < t + m; ++b)
+      R.ck_step[b] = F.step_index + (R.s_of(b) - t) + 1;
+    F.step_index += m;
+    run.bytes = m * step_bytes(F);
+    run.launch();
+  }
+}
+
+bool migrate_wave(ShotRun& R, cudaStream_t st) {
+  WaveShot W;
+  if (!wave_shot(R, W)) return false;
+  WaveRunner run(st);
+  wave_forward(run, R, W.whole);
+  bool together = wave_together(W) && !R.excitation && R.n_states > 1;
+  if (together && !R.rbuf[1].p) {
+    try {
+      R.rbuf[1] = DevBuf(R.rbuf[0].bytes, st);
+    } catch (const Error&) {   // no room for a second replay buffer: one after the other
+      cudaGetLastError();
+      together = false;
+    }
+  }
+  double lp = 0.0;
+  if (R.excitation) {
+    for (int b = 0; b < R.n_states; ++b)
+      for (int t = R.s_of(b); t < R.e_of(b); t += kWaveMaxSteps) {
+        run.begin();
+        wave_add_replay(run, R, W.alone, b, t, std::min(kWaveMaxSteps, R.e_of(b) - t));
+        run.launch();
+      }
+    for (int t = R.cfg.nt_spec - 1; t >= 0;) {
+      run.begin();
+      const int n = wave_add_backward(run, R, W.b, 0, t, std::min(kWaveMaxSteps, t + 1), lp);
+      run.launch();
+      t -= n;
+      if (lp > 0.0) wave_finish_lowpass(R, 0, t + 1, lp, st);
+    }
+    return true;
+  }
+  // replay position and backward position; the backward pass over block b
+  // runs once block b is replayed, the replay stays at most one block ahead
+  int rb = R.n_states - 1, rt = R.s_of(rb), bb = rb, bt = R.e_of(rb) - 1;
+  while (bb >= 0) {
+    const bool can_b = rb < bb;
+    const bool can_r = rb >= 0 && rb + (together ? 1 : 0) >= bb;
+    run.begin();
+    const bool do_b = can_b;
+    const bool do_r = can_r;
+    int nb = 0;
+    const int b_now = bb, t_now = bt;
+    lp = 0.0;
+    if (do_b) nb = wave_add_backward(run, R, W.b, bb, bt, std::min(kWaveMaxSteps, bt - R.s_of(bb) + 1), lp);
+    if (do_r) {
+      // beside a backward segment, as many steps as it has
+      const int left = R.e_of(rb) - rt;
+      const int nr = do_b ? std::min(left, std::max(nb, 1)) : std::min(left, kWaveMaxSteps);
+      wave_add_replay(run, R, do_b ? W.f : W.alone, rb, rt, nr);
+      rt += nr;
+      if (rt == R.e_of(rb)) {
+        --rb;
+        if (rb >= 0) rt = R.s_of(rb);
+      }
+    }
+    run.launch();
+    if (do_b) {
+      bt -= nb;
+      if (lp > 0.0) wave_finish_lowpass(R, b_now, t_now - nb + 1, lp, st);
+      if (bt < R.s_of(bb)) {
+        --bb;
+        if (bb >= 0) bt = R.e_of(bb) - 1;
+      }
+    }
+  }
+  return true;
 }
 
 // Plain driver: one shot, steps one after the other (imaging.py:255-331).
@@ -1617,6 +2128,12 @@ void migrate(Prop& F, Prop& B, const ertm_migrate_config& cfg, const float* wave
   cudaStream_t st = F.st;
   ShotRun R;
   prepare_run(R, F, B, cfg, wavelet, record, num_out, illum_out, rillum_out, st, 1);
+  if (migrate_wave(R, st)) {
+    CK(cudaGetLastError());
+    finish_run(R, st);
+    require_finite(R, st, "migrate");
+    return;
+  }
   const float* dw = R.wave.as<float>();
   auto fwd_step = [&](int t, const Epilogue& e) {
     if (R.fwd_unfused) {
@@ -2379,6 +2896,13 @@ int32_t ertm_set_lane_assign(int32_t mode) {
   });
 }
 
+int32_t ertm_set_wave(int32_t mode) {
+  return guarded([&] {
+    REQUIRE(mode >= 0 && mode <= 2, "multi-step launches: 0 (automatic), 1 (never) or 2 (wherever they fit)");
+    g_wave.store(mode);
+  });
+}
+
 int32_t ertm_set_tma(int32_t enable) {
   return guarded([&] { g_tma.store(enable ? 1 : 0); });
 }
@@ -2722,16 +3246,24 @@ int32_t ertm_forward(void* prop, int32_t nt, const float* amps, int32_t n_comp, 
     const bool sampling = n > 0 && n_comp > 0;
     DevBuf o(sampling ? (size_t)n_comp * nt * n * 4 : 0, P.st);
     SampleSet S{};
+    std::vector<SamplePlanHost*> plans;
     if (sampling) {
       S.count = n_comp;
       for (int c = 0; c < n_comp; ++c) {
         SamplePlanHost& sp = sample_plan(P, comps[c]);
+        plans.push_back(&sp);
         S.plan[c] = SamplePlanDev{n, sp.kind, sp.slot, 0, sp.cell.as<int32_t>(), sp.valid.as<uint8_t>(),
                                   sp.w.as<double>(), o.as<float>() + (size_t)c * nt * n};
       }
     }
     DevBuf dwave(amps ? (size_t)nt * 4 : 0, P.st);
     if (amps) upload(dwave.p, amps, (size_t)nt * 4, P.st);
+    if (forward_wave(P, nt, amps ? dwave.as<float>() : nullptr, S, plans)) {
+      REQUIRE(!(read_status(P, P.st) & STATUS_STALLED), "a wait between the CTAs of a launch ran out");
+      if (sampling) CK(cudaMemcpyAsync(out, o.p, o.bytes, cudaMemcpyDefault, P.st));
+      CK(cudaStreamSynchronize(P.st));
+      return;
+    }
     for (int t = 0; t < nt; ++t) {
       if (amps) step_once(P, 0.0, dwave.as<float>(), t);
       else step_once(P, 0.0);

@@ -78,6 +78,8 @@ struct DevProp {
 // it writes a NaN or an infinity (an unstable or overflowing run); hosts read
 // the word between steps and fail that run alone.
 constexpr uint32_t STATUS_NONFINITE = 1u;
+// A bounded wait between the CTAs of a multi-step launch ran out (wave_kernel.cuh).
+constexpr uint32_t STATUS_STALLED = 2u;
 
 __device__ __forceinline__ bool nonfinite4(const float4& v) {
   // NaN fails every comparison; |±inf| exceeds the largest finite float
@@ -137,6 +139,13 @@ struct StepWork {
   Epilogue epi;
 };
 constexpr int STEP_PEAK = 1;        // visco: reduce max|p| into DevProp::peak
+
+// Amplitude-cap state of a compensated viscoacoustic propagator.
+struct StabState {
+  double ref_amp;   // reference amplitude: running max|p| over steps < 30
+  int32_t clipped;  // amplitude-cap events
+  int32_t pad_;
+};
 
 // The works of one launch, passed by value in the kernel parameters: one work
 // (plain stepping) or up to N (batched ticks; blocks find their work by binary

@@ -158,6 +158,11 @@ int32_t ertm_set_march(int32_t enable);
  * (default): tiles.  Takes effect while ertm_set_march is non-zero.  Results
  * do not depend on it. */
 int32_t ertm_set_march_stress(int32_t enable);
+
+/* Multi-step launches (wavefields kept in shared memory over many steps):
+ * 0 where they are expected to be faster, 1 never, 2 wherever they fit.
+ * Results are identical in every mode. */
+int32_t ertm_set_wave(int32_t mode);
 /* Online autotuning of batched ticks (default on): the first ticks of each
  * group shape (engine, order, works, size class) try tile heights 8/16/32,
  * split off/on and one or two lanes, timed with CUDA events; the fastest is
