@@ -445,6 +445,20 @@ struct InjectPlanHost {
   }
 };
 
+// How a propagator is split over at most `ncta` CTAs.
+struct WavePlan {
+  int px = 0, pz = 0;
+  int cells = 1;      // neighbouring cells of a thread's block
+  int thmax = 0, n_src = 0, n_acc = 0;
+  std::vector<int16_t> cut;
+  bool res = false;
+  int pad = 8;        // halo-field row padding (wave_layout)
+  int smem = 0;       // bytes
+  int64_t half = 0;   // exchange units per CTA and phase
+  bool ok() const { return px > 0; }
+  int ctas() const { return px * pz; }
+};
+
 struct Prop {
   ertm_prop_config cfg{};
   DevProp h{};
@@ -465,6 +479,7 @@ struct Prop {
   std::vector<float> host_kr;    // K_R copy for the ε-injection weights (lazy)
   size_t fe = 0;                 // field pitch in the state and coefficient blocks (floats)
   int n_coef = 0;
+  mutable std::map<std::array<int, 4>, WavePlan> waves;    // multi-step splits (see wave_plan)
   mutable std::map<int, std::array<CUtensorMap, 3>> tma;   // tensor maps per tile height (see prop_tma)
   DevBuf tma_dev;                // the same maps in device memory for tile heights 8, 16, 32
   // complex work arrays of the compensated viscoacoustic low-pass (nzp·nxp each)
@@ -1650,27 +1665,22 @@ int sm_count() {
   return n;
 }
 
-// How a propagator is split over at most `ncta` CTAs.
-struct WavePlan {
-  int px = 0, pz = 0, cells = 1;   // cells: per thread and pass
-  bool res = false;
-  int pad = 8;        // halo-field row padding (wave_layout)
-  int smem = 0;       // bytes
-  int64_t half = 0;   // exchange units per CTA and phase
-  bool ok() const { return px > 0; }
-  int ctas() const { return px * pz; }
+// What a work does besides stepping, for its shared memory: epilogue fields
+// (P, S), stored source fields read, imaging sums that could be resident.
+struct WaveNeeds {
+  int n_epi = 0, n_src = 0, n_acc = 0;
 };
 
 // Largest shared-memory need of a split, in bytes.
-int wave_smem(const DevProp& h, const WavePlan& p, int n_epi) {
-  const int ng = (h.nxp + 3) / 4;
+int wave_smem(const DevProp& h, const WavePlan& p, const WaveNeeds& n) {
   int most = 0;
   for (int c = 0; c < p.px * p.pz; ++c) {
-    const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c);
+    const WaveTile t = wave_tile(p.cut.data(), p.pz, p.px, c);
     int f, nsx, nsz;
     wave_strip(4 * t.g0, std::min(4 * (t.g0 + t.gw), h.nxp), h.nxp, h.npx_l, h.npx_r, f, nsx);
     wave_strip(t.i0, t.i0 + t.th, h.nzp, h.npz_t, h.npz_b, f, nsz);
-    const WaveLayout y = wave_layout(h.engine == ENGINE_ELASTIC, h.engine == ENGINE_VISCO, h.L, p.res, p.pad, t.th, t.gw, nsx, nsz, n_epi);
+    const WaveLayout y = wave_layout(h.engine == ENGINE_ELASTIC, h.engine == ENGINE_VISCO, h.L, p.res, p.pad, t.th,
+                                     t.gw, nsx, nsz, n.n_epi, p.n_src, p.n_acc);
     most = std::max(most, y.total * 4);
   }
   return most;
@@ -1681,35 +1691,104 @@ bool wave_supported(const DevProp& h) {
          (h.engine != ENGINE_VISCO || h.L <= kRelaxUnroll);
 }
 
-WavePlan wave_plan(const DevProp& h, int ncta, int n_epi) {
+// Cuts of n positions into k parts of about equal weight, each at least
+// `least` long; position q weighs weight(q).
+template <class F>
+void wave_cuts(int n, int k, int least, F&& weight, int16_t* cut) {
+  double total = 0.0;
+  for (int q = 0; q < n; ++q) total += weight(q);
+  double sum = 0.0;
+  int at = 0, first = 0;
+  cut[0] = 0;
+  for (int c = 0; c < k; ++c) {
+    const int last = n - least * (k - 1 - c);   // leave the later parts their least
+    while (at < last && (at - first < least || c + 1 == k || sum + 0.5 * weight(at) < total * (c + 1) / k)) {
+      sum += weight(at);
+      ++at;
+    }
+    cut[c + 1] = (int16_t)at;
+    first = at;
+  }
+}
+
+// Split over at most `ncta` CTAs.  Measured over px = 5 … 24 and strip weights
+// 0 … 2 on five grids: CTAs about 2.2 times as wide as tall are within 2 % of
+// the best, and so is a weight of 1.6 for CPML strips (their cells take the
+// general form and memory updates) with two cells a thread; with one cell a
+// thread (small grids, one pass of 512) 0.4.  Elastic 401×601 (µs a step):
+// 6.9 so, 7.9 with equal cuts, 11.6 the worst; acoustic 301×201 3.4 with one
+// cell a thread, 4.6 with two.  Imaging sums that do not fit in shared memory
+// cost about two round trips to L2 a step, coefficients that do not fit more.
+WavePlan make_wave_plan(const DevProp& h, int ncta, const WaveNeeds& n) {
   WavePlan best;
   if (!wave_supported(h)) return best;
-  const int ng = (h.nxp + 3) / 4;
+  const int ng = (h.nxp + 3) / 4, nx = h.engine == ENGINE_ELASTIC ? 2 : 1;
+  ncta = std::min(ncta, WAVE_MAX_CUTS - 4);
+  const double ideal = std::sqrt((double)h.nxp * ncta / (2.2 * h.nzp));
+  // cells per thread and pass; a split of one pass (WAVE_NT blocks a CTA at
+  // most) is cut for that rather than by weight
+  const double avg = (double)h.nzp * 4 * ng / (0.93 * WAVE_NT * ncta);
+  const int cells = avg <= 1.0 ? 1 : 2;
+  const bool single = avg <= 2.0;
   double cost = 0.0;
-  for (int px = 1; px <= std::min(ncta, ng); ++px) {
+  for (const double strip : {single ? 0.4 : 1.6, 0.8, 0.0})
+  for (int px = std::max(1, std::min(ng, (int)ideal) - 2); px <= std::min({ncta, ng, (int)ideal + 3}); ++px) {
     const int pz = std::min(ncta / px, h.nzp / WAVE_HALO);
     if (pz < 1) continue;
-    const int th = (h.nzp + pz - 1) / pz, gw = (ng + px - 1) / px;
-    const double c = (double)(th + 2 * WAVE_HALO) * (4 * gw + 2 * WAVE_HALO);
-    if (best.px == 0 || c < cost) {
-      best.px = px;
-      best.pz = pz;
+    auto row_w = [&](int i) { return i < h.npz_t || i >= h.nzp - h.npz_b ? 1.0 + strip : 1.0; };
+    auto col_w = [&](int g) {
+      int s = 0;
+      for (int j = 4 * g; j < 4 * g + 4; ++j) s += j < h.npx_l || (j >= h.nxp - h.npx_r && j < h.nxp) ? 1 : 0;
+      return 4.0 + strip * s;
+    };
+    WavePlan p;
+    p.px = px;
+    p.pz = pz;
+    p.cells = cells;
+    p.cut.resize(pz + px + 2);
+    wave_cuts(h.nzp, pz, WAVE_HALO, row_w, p.cut.data());
+    wave_cuts(ng, px, 1, col_w, p.cut.data() + pz + 1);
+    int gw = 0, most = 0;
+    for (int c = 0; c < p.ctas(); ++c) {
+      const WaveTile t = wave_tile(p.cut.data(), pz, px, c);
+      p.thmax = std::max(p.thmax, t.th);
+      gw = std::max(gw, t.gw);
+      most = std::max(most, t.th * t.gw * 4);
+    }
+    p.half = (int64_t)2 * nx * p.thmax + (int64_t)2 * nx * 4 * gw;
+    // the most that fits: resident coefficients first, then resident sums,
+    // then conflict-free rows
+    bool fits = false;
+    for (int k = 0; k < 8 && !fits; ++k) {
+      p.n_acc = (k & 2) == 0 ? n.n_acc : 0;
+      p.n_src = p.n_acc ? n.n_src : 0;
+      p.pad = (k & 1) == 0 ? 32 : 8;
+      p.res = k < 4;
+      p.smem = wave_smem(h, p, n);
+      fits = p.smem <= kWaveSmemMax;
+    }
+    if (!fits) continue;
+    // relative cost of a step: SMs left idle, the shape, equal cuts (measured
+    // 14 % with two cells a thread), a second pass of a few cells, sums and
+    // coefficients that do not fit
+    const double c = (double)ncta / p.ctas() * (1.0 + 0.03 * std::fabs(px - ideal)) *
+                     (single ? 1.0 + 0.05 * std::fabs(strip - 0.4) : 1.0 + 0.09 * (1.6 - strip)) *
+                     (single && most > WAVE_NT * cells ? 1.3 : 1.0) * (p.n_acc < n.n_acc ? 1.25 : 1.0) * (p.res ? 1.0 : 2.0);
+    if (!best.ok() || c < cost) {
+      best = p;
       cost = c;
     }
   }
-  if (!best.ok()) return best;
-  const int th = (h.nzp + best.pz - 1) / best.pz, gw = (ng + best.px - 1) / best.px;
-  const int nx = h.engine == ENGINE_ELASTIC ? 2 : 1;
-  best.half = (int64_t)2 * nx * th + (int64_t)2 * nx * 4 * gw;
-  best.cells = th * 4 * gw <= WAVE_NT ? 1 : 2;
-  for (int k = 0; k < 4; ++k) {
-    best.res = k < 2;
-    best.pad = (k & 1) == 0 ? 32 : 8;
-    best.smem = wave_smem(h, best, n_epi);
-    if (best.smem <= kWaveSmemMax) return best;
-  }
-  best.px = 0;
   return best;
+}
+
+// The propagator's split, kept with it (0.1–0.5 ms to make; a function of the
+// grid and the needs alone).
+const WavePlan& wave_plan(const Prop& P, int ncta, const WaveNeeds& n) {
+  const std::array<int, 4> key{ncta, n.n_epi, n.n_src, n.n_acc};
+  auto it = P.waves.find(key);
+  if (it == P.waves.end()) it = P.waves.emplace(key, make_wave_plan(P.h, ncta, n)).first;
+  return it->second;
 }
 
 // Exchange buffers of one driver call.  Epochs only grow, so words of earlier
@@ -1739,6 +1818,10 @@ struct WaveRunner {
     w.px = p.px;
     w.pz = p.pz;
     w.pad = p.pad;
+    w.thmax = p.thmax;
+    w.n_src = p.n_src;
+    w.n_acc = p.n_acc;
+    std::copy(p.cut.begin(), p.cut.end(), w.cut);
     w.n_steps = n_steps;
     w.sign = 1;
     grid += p.ctas();
@@ -1776,15 +1859,10 @@ struct WaveOwner {
   std::vector<int> tr, tc;
   int px;
   WaveOwner(const DevProp& h, const WavePlan& p) : tr(h.nzp), tc((h.nxp + 3) / 4), px(p.px) {
-    const int ng = (int)tc.size();
-    for (int c = 0; c < p.pz; ++c) {
-      const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c * p.px);
-      for (int i = 0; i < t.th; ++i) tr[t.i0 + i] = c;
-    }
-    for (int c = 0; c < p.px; ++c) {
-      const WaveTile t = wave_tile(h.nzp, ng, p.pz, p.px, c);
-      for (int g = 0; g < t.gw; ++g) tc[t.g0 + g] = c;
-    }
+    for (int c = 0; c < p.pz; ++c)
+      for (int i = p.cut[c]; i < p.cut[c + 1]; ++i) tr[i] = c;
+    for (int c = 0; c < p.px; ++c)
+      for (int g = p.cut[p.pz + 1 + c]; g < p.cut[p.pz + 2 + c]; ++g) tc[g] = c;
   }
   int of(int i, int j) const { return tr[i] * px + tc[j / 4]; }
 };
@@ -1796,7 +1874,7 @@ DevBuf wave_upload(const void* data, size_t bytes, cudaStream_t st) {
 }
 
 const WaveInjectHost& wave_inject(const Prop& P, InjectPlanHost& plan, const WavePlan& p) {
-  auto it = plan.wave.find({p.px, p.pz});
+  auto it = plan.wave.find({p.px, p.pz});   // a grid's cuts depend on these alone
   if (it != plan.wave.end()) return it->second;
   const WaveOwner own(P.h, p);
   const int n = plan.n_cells, nc = p.ctas();
@@ -1888,7 +1966,7 @@ bool wave_wanted(const WavePlan& p) {
 bool forward_wave(Prop& P, int nt, const float* dwave, const SampleSet& S, const std::vector<SamplePlanHost*>& comps) {
   const bool comp = P.h.engine == ENGINE_VISCO && P.cfg.compensation;
   if (nt < 2 || comp) return false;
-  const WavePlan p = wave_plan(P.h, sm_count(), 0);
+  const WavePlan p = wave_plan(P, sm_count(), {});
   if (!wave_wanted(p)) return false;
   const int n = S.count ? S.plan[0].n : 0;
   const int64_t stride = 4 * (int64_t)S.count * n;
@@ -1941,18 +2019,27 @@ bool wave_shot(const ShotRun& R, WaveShot& W) {
   if (R.fwd_unfused) return false;
   if (F.h.engine == ENGINE_VISCO && F.cfg.compensation) return false;
   const int n = sm_count();
-  const int nf = 1 + (F.h.engine == ENGINE_ELASTIC && R.need_src[1] ? 1 : 0);
-  const int nb = 1 + (F.h.engine == ENGINE_ELASTIC && R.need_rcv_s ? 1 : 0);
-  W.whole = wave_plan(F.h, n, 0);
+  WaveNeeds nf, nb;
+  if (F.h.engine == ENGINE_ELASTIC) {   // pressure engines image p where it is
+    nf.n_epi = R.need_src[1] ? 2 : 1;
+    nb.n_epi = R.need_rcv_s ? 2 : 1;
+  }
+  if (!R.excitation) {
+    nb.n_src = R.n_src;
+    for (int k = 0; k < R.cfg.n_images; ++k)
+      nb.n_acc += 1 + (R.want_ill && R.base.ill[k] ? 1 : 0) + (R.want_ril && R.base.ril[k] ? 1 : 0);
+  }
+  W.whole = wave_plan(F, n, {});
   if (!wave_wanted(W.whole)) return false;
   // side by side on half the SMs each; one after the other on all of them
   // when half the SMs cannot hold a propagator's resident arrays
-  W.alone = wave_plan(F.h, n, nf);
-  W.f = wave_plan(F.h, n / 2, nf);
-  W.b = wave_plan(B.h, n / 2, nb);
-  if (!W.f.ok() || !W.b.ok() || W.f.res != W.b.res || !W.f.res || W.f.cells != W.b.cells) {
+  W.alone = wave_plan(F, n, nf);
+  W.f = wave_plan(F, n / 2, nf);
+  W.b = wave_plan(B, n / 2, nb);
+  if (!W.f.ok() || !W.b.ok() || W.f.res != W.b.res || !W.f.res || W.f.cells != W.b.cells ||
+      (W.b.n_acc < nb.n_acc && wave_plan(B, n, nb).n_acc == nb.n_acc)) {
     W.f = W.alone;
-    W.b = wave_plan(B.h, n, nb);
+    W.b = wave_plan(B, n, nb);
   }
   return wave_wanted(W.alone) && wave_wanted(W.f) && wave_wanted(W.b);
 }

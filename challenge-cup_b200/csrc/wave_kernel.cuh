@@ -26,13 +26,18 @@
 //    at the end of their step.
 //
 // What bounds a step now is the chain publish → neighbour's poll → sync (about
-// 1700 cycles, twice) plus the two phases of the slowest CTA (edge CTAs with
-// CPML strips).  512 threads (128 registers, no spills) beat 640, 768 and 1024
-// (64 registers): 1500 acoustic steps of 301×201 with 151 receivers take
-// 4.6 ms against 5.2, 5.4 and 5.7 ms.  Against two or three launches a step:
-// that run 24.9 → 4.6 ms, 1000 elastic steps of 401×601 20.9 → 7.9 ms, a
-// 1500-step acoustic migration 63.3 → 13.4 ms, an 800-step PP/PS migration of
-// 401×601 50.7 → 27.1 ms.
+// 1700 cycles, twice) plus the two phases of the slowest CTA; a phase is a
+// pass of 512 blocks of one or two cells at 750 (straight-line form) to 2200
+// cycles (general form) of latency plus 0.8–2 cycles a cell of issue and
+// shared-memory bandwidth.  So an edge CTA runs the straight-line form where
+// it can, cuts weigh CPML strips, and imaging sums stay in shared memory for
+// the launch where they fit (1000 elastic steps of 401×601: 7.9 → 6.7 ms,
+// an 800-step PP/PS migration 27.1 → 24.5 ms).  512 threads (128 registers, no
+// spills) beat 640, 768 and 1024 (64 registers): 1500 acoustic steps of 301×201
+// with 151 receivers 4.6 ms against 5.2, 5.4 and 5.7 ms; 2 × 2 cells a thread
+// were no faster than 2 × 1.  Against two or three launches a step: that run
+// 24.9 → 4.6 ms, the elastic one 20.9 → 6.7 ms, a 1500-step acoustic migration
+// 63.3 → 13.7 ms, the PP/PS migration 50.7 → 24.5 ms.
 //
 // Every wait is bounded: when a wait runs out the CTA sets STATUS_STALLED and
 // leaves; its neighbours' waits then run out too.  Co-residency is the
@@ -53,20 +58,22 @@ constexpr int WAVE_MAX_WORKS = 16;
 constexpr int WAVE_SPIN_LIMIT = 1 << 20;   // polls of one packet (about a second)
 constexpr int WAVE_HALO = 4;
 
-// Rows [i0, i0 + th) and column groups [g0, g0 + gw) of CTA c of a pz × px split.
+// Rows [i0, i0 + th) and column groups [g0, g0 + gw) of CTA c of a pz × px
+// split with row cuts cut[0 … pz] and column-group cuts cut[pz + 1 …].
 struct WaveTile {
   int i0, th, g0, gw, tr, tc;
 };
-__host__ __device__ inline WaveTile wave_tile(int nzp, int ng, int pz, int px, int c) {
+__host__ __device__ inline WaveTile wave_tile(const int16_t* cut, int pz, int px, int c) {
   WaveTile t;
   t.tr = c / px;
   t.tc = c - t.tr * px;
-  t.i0 = (int)((long long)t.tr * nzp / pz);
-  t.th = (int)((long long)(t.tr + 1) * nzp / pz) - t.i0;
-  t.g0 = (int)((long long)t.tc * ng / px);
-  t.gw = (int)((long long)(t.tc + 1) * ng / px) - t.g0;
+  t.i0 = cut[t.tr];
+  t.th = cut[t.tr + 1] - t.i0;
+  t.g0 = cut[pz + 1 + t.tc];
+  t.gw = cut[pz + 2 + t.tc] - t.g0;
   return t;
 }
+constexpr int WAVE_MAX_CUTS = 160;   // pz + px + 2 of a split over up to 156 CTAs
 
 // Strip columns / rows of [lo, hi) in ψ-array coordinates: first index and count.
 __host__ __device__ inline void wave_strip(int lo, int hi, int n, int a, int b, int& first, int& count) {
@@ -87,6 +94,8 @@ struct WaveLayout {
   int cell, cell_n;      // per-cell arrays, floats per array
   int qidx;              // viscoacoustic Q index bytes
   int epi;               // P (and S) of the last step for the epilogue
+  int src;               // stored source fields of the last step
+  int acc;               // imaging sums, two floats a cell each
   int psix, psix_n;      // x-strip memories (pitch nsx), floats per term
   int psiz, psiz_n;      // z-strip memories (pitch cw), floats per term
   int col, row;          // per column / row: profile a, b, strip index and flags
@@ -100,7 +109,7 @@ __host__ __device__ inline int wave_r4(int n) { return (n + 3) / 4 * 4; }
 // the halo; with 32 the rows' first cells continue the bank sequence of the
 // cells before them, so a warp that spans rows has no bank conflicts.
 __host__ __device__ inline WaveLayout wave_layout(bool elastic, bool visco, int L, bool res, int pad, int th, int gw,
-                                                  int nsx, int nsz, int n_epi) {
+                                                  int nsx, int nsz, int n_epi, int n_src, int n_acc) {
   WaveLayout y;
   const int nf = elastic ? 5 : 3, nx = elastic ? 2 : 1, n_psi = elastic ? 4 : 2;
   y.cw = 4 * gw;
@@ -117,6 +126,10 @@ __host__ __device__ inline WaveLayout wave_layout(bool elastic, bool visco, int 
   o += res && visco ? wave_r4(th * gw) : 0;   // one byte per cell
   y.epi = o;
   o += n_epi * y.cell_n;
+  y.src = o;
+  o += n_src * y.cell_n;
+  y.acc = o;
+  o += 2 * n_acc * y.cell_n;
   y.psix = o;
   y.psix_n = res ? wave_r4(th * nsx) : 0;
   o += n_psi * y.psix_n;
@@ -168,6 +181,34 @@ __host__ __device__ inline WaveUnit wave_unit(bool elastic, int phase, int u, co
   return q;
 }
 
+// Blocks (C neighbouring cells) of a CTA whose cells are all physical, clear of
+// strips and of the free surface: rows [b0, b1) × block columns [v0, v1) of
+// nb × nv.  A CTA of one pass takes one form for all its blocks: two passes
+// would cost more than the general form does.
+struct WaveInner {
+  int nb, nv, b0, b1, v0, v1;
+  __host__ __device__ int inner() const { return (b1 - b0) * (v1 - v0); }
+  __host__ __device__ int frame() const { return nb * nv - inner(); }
+};
+template <class GEO>
+__host__ __device__ inline WaveInner wave_inner(const GEO& G, const WaveTile& T, int C) {
+  auto lo = [](int a, int b) { return a < b ? a : b; };
+  auto hi = [](int a, int b) { return a > b ? a : b; };
+  const int i0 = T.i0, j0 = 4 * T.g0, cw = 4 * T.gw;
+  const int lo_i = hi(hi(G.pad, G.npz_t), G.free_surface ? G.pad + 1 : 0) - i0;
+  const int hi_i = lo(G.pad + G.nz, G.nzp - G.npz_b) - i0;
+  const int lo_j = hi(G.pad, G.npx_l) - j0, hi_j = lo(G.pad + G.nx, G.nxp - G.npx_r) - j0;
+  WaveInner I;
+  I.nb = T.th;
+  I.nv = cw / C;
+  I.b0 = lo(hi(lo_i, 0), I.nb);
+  I.b1 = hi(I.b0, lo(hi(hi_i, 0), T.th));
+  I.v0 = lo((hi(lo_j, 0) + C - 1) / C, I.nv);
+  I.v1 = hi(I.v0, lo(hi(hi_j, 0), cw) / C);
+  if (I.b0 == I.b1 || I.v0 == I.v1 || (I.frame() > 0 && I.nb * I.nv <= WAVE_NT)) I.b0 = I.b1 = I.v0 = I.v1 = 0;
+  return I;
+}
+
 constexpr int WAVE_STAB = 1;        // compensated viscoacoustic amplitude cap inside the launch
 constexpr int WAVE_SKIP_LAST = 2;   // the last step's epilogue runs after the launch (a low-pass comes first)
 
@@ -196,9 +237,11 @@ struct WaveSample {
 
 struct WaveWork {
   const DevProp* prop;
-  int32_t cta0, px, pz;
+  int32_t cta0, px, pz, thmax;       // thmax: the tallest CTA
+  int16_t cut[WAVE_MAX_CUTS];        // see wave_tile
   int32_t n_steps, t0, sign;         // time index of step k: t0 + sign·k
   int32_t flags, pad;                // WAVE_* bits; halo-field row padding (wave_layout)
+  int32_t n_src, n_acc;              // stored source fields staged and imaging sums kept in shared memory
   uint32_t epoch;                    // epochs epoch + 1 … epoch + 2·n_steps
   int32_t start_step;                // cross-correlate from this time on
   const float* wavelet;              // nullptr: no source
@@ -235,6 +278,7 @@ __device__ __forceinline__ void wave_put(uint64_t* p, int64_t plane, const float
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n" ::"l"(p + plane), "l"(c), "l"(d) : "memory");
 }
 __device__ __forceinline__ bool wave_get(const uint64_t* p, int64_t plane, uint32_t e, float4& v) {
+#pragma unroll 1
   for (int it = 0; it < WAVE_SPIN_LIMIT; ++it) {
     uint64_t a, b, c, d;
     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n" : "=l"(a), "=l"(b) : "l"(p) : "memory");
@@ -280,7 +324,7 @@ __device__ __forceinline__ void xwin(const float* p, float (&v)[8 + C]) {
     for (int k = 0; k < 9; ++k) v[k] = p[k - 4];
   }
 }
-// rows −4 … 4; row 0 at index 4 (rows a stencil does not use are not loaded)
+// rows −4 … 4; row 0 at index 4 (rows no stencil uses are not loaded)
 template <int C>
 __device__ __forceinline__ void zwin(const float* p, int W, float (&z)[C][9]) {
 #pragma unroll
@@ -306,7 +350,7 @@ __device__ __forceinline__ float wave_minus(const float* f, int o) { return wave
 __device__ __forceinline__ bool nonfinite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 
 // C neighbouring cells through the work's epilogue at time t (run_epilogue's
-// arithmetic); float64 sums are loaded for all the cells before any is stored.
+// arithmetic), except the imaging condition with float64 sums.
 template <int C>
 __device__ __forceinline__ void wave_epilogue(const WaveWork& w, int t, ptrdiff_t c0, const bool (&ok)[C],
                                               size_t npix, const float (&pv)[C], const float (&sv)[C]) {
@@ -327,43 +371,16 @@ __device__ __forceinline__ void wave_epilogue(const WaveWork& w, int t, ptrdiff_
       s[0][c] = (ok[c] && E.src[0]) ? E.src[0][at + c] : 0.f;
       s[1][c] = (ok[c] && E.src[1]) ? E.src[1][at + c] : 0.f;
     }
-    if (!E.kahan) {
-      double v[3][MAX_EPI_IMAGES][C];
 #pragma unroll
-      for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
-        if (k >= E.n_images) break;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          if (!ok[c]) continue;
-          if (E.illum && E.ill[k]) v[0][k][c] = E.ill[k][c0 + c];
-          if (E.rillum && E.ril[k]) v[1][k][c] = E.ril[k][c0 + c];
-          if (cross) v[2][k][c] = E.num[k][c0 + c];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
-        if (k >= E.n_images) break;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          if (!ok[c]) continue;
-          const float a = E.src_slot[k] ? s[1][c] : s[0][c];
-          const float r = E.rcv_wave[k] ? sv[c] : pv[c];
-          if (E.illum && E.ill[k]) E.ill[k][c0 + c] = dadd(v[0][k][c], (double)fmul(a, a));
-          if (E.rillum && E.ril[k]) E.ril[k][c0 + c] = dadd(v[1][k][c], (double)fmul(r, r));
-          if (cross) E.num[k][c0 + c] = dadd(v[2][k][c], (double)fmul(a, r));
-        }
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        if (!ok[c]) continue;
-        for (int k = 0; k < E.n_images; ++k) {
-          const float a = E.src_slot[k] ? s[1][c] : s[0][c];
-          const float r = E.rcv_wave[k] ? sv[c] : pv[c];
-          if (E.illum && E.ill[k]) acc_term(E.ill[k], 1, c0 + c, npix, fmul(a, a));
-          if (E.rillum && E.ril[k]) acc_term(E.ril[k], 1, c0 + c, npix, fmul(r, r));
-          if (cross) acc_term(E.num[k], 1, c0 + c, npix, fmul(a, r));
-        }
+    for (int c = 0; c < C; ++c) {
+      if (!ok[c]) continue;
+#pragma unroll 1
+      for (int k = 0; k < E.n_images; ++k) {
+        const float a = E.src_slot[k] ? s[1][c] : s[0][c];
+        const float r = E.rcv_wave[k] ? sv[c] : pv[c];
+        if (E.illum && E.ill[k]) acc_term(E.ill[k], 1, c0 + c, npix, fmul(a, a));
+        if (E.rillum && E.ril[k]) acc_term(E.ril[k], 1, c0 + c, npix, fmul(r, r));
+        if (cross) acc_term(E.num[k], 1, c0 + c, npix, fmul(a, r));
       }
     }
   } else if (E.kind == EPI_EXC_TRACK) {
@@ -381,6 +398,7 @@ __device__ __forceinline__ void wave_epilogue(const WaveWork& w, int t, ptrdiff_
     for (int c = 0; c < C; ++c) {
       if (!ok[c] || E.peak_step[c0 + c] != t) continue;
       const double a = (double)E.running[c0 + c];
+#pragma unroll 1
       for (int k = 0; k < E.n_images; ++k) {
         const float r = E.rcv_wave[k] ? sv[c] : pv[c];
         E.num[k][c0 + c] = dadd(E.num[k][c0 + c], dmul(a, (double)r));
@@ -390,12 +408,147 @@ __device__ __forceinline__ void wave_epilogue(const WaveWork& w, int t, ptrdiff_
   }
 }
 
+// The imaging condition with float64 sums in global memory for U pieces of C
+// cells: two sums of every piece are loaded together before any is stored,
+// so a step waits for one or two round trips to L2 instead of one per piece
+// and sum.
+template <int U, int C>
+struct WavePieces {
+  ptrdiff_t at[U];       // physical offset of the first cell
+  unsigned ok;           // bit u·C + c: the cell is physical
+  float pv[U][C], sv[U][C];
+};
+template <int U, int C>
+__device__ __forceinline__ void wave_image_global(const WaveWork& w, int t, const WavePieces<U, C>& K) {
+  const Epilogue& E = w.epi;
+  const bool cross = t >= w.start_step;
+  const ptrdiff_t slot = (ptrdiff_t)(t - w.slot_t) * w.slot_floats;
+  float s[2][U][C];
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        s[n][u][c] = (E.src[n] && (K.ok >> (u * C + c) & 1)) ? E.src[n][slot + K.at[u] + c] : 0.f;
+  // term kinds: 0 S², 1 R², 2 S·R
+  auto term = [&](int kind, int k, int u, int c) {
+    const float a = E.src_slot[k] ? s[1][u][c] : s[0][u][c];
+    const float r = E.rcv_wave[k] ? K.sv[u][c] : K.pv[u][c];
+    return (double)(kind == 0 ? fmul(a, a) : (kind == 1 ? fmul(r, r) : fmul(a, r)));
+  };
+  double* p0 = nullptr;
+  int kind0 = 0, k0 = 0;
+  auto run = [&](double* p, int kind, int k) {   // pairs up the sums
+    if (!p0) {
+      p0 = p;
+      kind0 = kind;
+      k0 = k;
+      return;
+    }
+    double v0[U][C], v1[U][C];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (K.ok >> (u * C + c) & 1) {
+          v0[u][c] = p0[K.at[u] + c];
+          if (p) v1[u][c] = p[K.at[u] + c];
+        }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (K.ok >> (u * C + c) & 1) {
+          p0[K.at[u] + c] = dadd(v0[u][c], term(kind0, k0, u, c));
+          if (p) p[K.at[u] + c] = dadd(v1[u][c], term(kind, k, u, c));
+        }
+    p0 = nullptr;
+  };
+#pragma unroll 1
+  for (int k = 0; k < E.n_images; ++k) {
+#pragma unroll 1
+    for (int kind = 0; kind < 3; ++kind) {
+      double* const p = kind == 0 ? (E.illum ? E.ill[k] : nullptr) : (kind == 1 ? (E.rillum ? E.ril[k] : nullptr)
+                                                                                : (cross ? E.num[k] : nullptr));
+      if (p) run(p, kind, k);
+    }
+  }
+  if (p0) run(nullptr, 0, 0);
+}
+
+// The imaging condition with the sums resident (see wave_epilogue): sums of
+// the thread's cells at offset o of the tile, source values staged.
+template <int C>
+__device__ __forceinline__ void wave_image_resident(const Epilogue& E, bool cross, float* acc, const float* src, int CN,
+                                                    int o, const float (&pv)[C], const float (&sv)[C]) {
+  float s[2][C] = {};
+  int q = 0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (E.src[k]) ldv<C>(src + (q++) * CN + o, s[k]);
+  auto add = [&](bool live, const float (&term)[C]) {
+    if (live) {
+      if (!E.kahan) {
+        double* const a = reinterpret_cast<double*>(acc) + o;
+#pragma unroll
+        for (int c = 0; c < C; ++c) a[c] = dadd(a[c], (double)term[c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const float y = fsub(term[c], acc[CN + o + c]), v = acc[o + c], t = fadd(v, y);
+          acc[CN + o + c] = fsub(fsub(t, v), y);
+          acc[o + c] = t;
+        }
+      }
+    }
+    acc += 2 * CN;
+  };
+#pragma unroll 1
+  for (int k = 0; k < E.n_images; ++k) {
+    float a[C], r[C], t[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      a[c] = E.src_slot[k] ? s[1][c] : s[0][c];
+      r[c] = E.rcv_wave[k] ? sv[c] : pv[c];
+    }
+    if (E.illum && E.ill[k]) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) t[c] = fmul(a[c], a[c]);
+      add(true, t);
+    }
+    if (E.rillum && E.ril[k]) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) t[c] = fmul(r[c], r[c]);
+      add(true, t);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) t[c] = fmul(a[c], r[c]);
+    add(cross, t);
+  }
+}
+
+// The work's imaging sums in the order wave_image_resident walks them.
+template <class F>
+__device__ __forceinline__ void wave_each_sum(const Epilogue& E, F&& f) {
+  int q = 0;
+#pragma unroll 1
+  for (int k = 0; k < E.n_images; ++k) {
+    if (E.illum && E.ill[k]) f(q++, E.ill[k]);
+    if (E.rillum && E.ril[k]) f(q++, E.ril[k]);
+    f(q++, E.num[k]);
+  }
+}
+
+__device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+
 // Column and row table entries: profile values, strip index (−1: none) with
 // flags.
 constexpr int WAVE_IN = 1;        // the derivative across this axis is inside the stencil's range
 constexpr int WAVE_OK = 2;        // column of the padded grid (not row padding)
-constexpr int WAVE_SRC = 4;       // the source's column / row
-constexpr int WAVE_SURFACE = 8;   // the free-surface row
+constexpr int WAVE_SURFACE = 4;   // the free-surface row
 __device__ __forceinline__ int wave_strip_of(const float4& t) { return __float_as_int(t.z); }
 __device__ __forceinline__ int wave_flags_of(const float4& t) { return __float_as_int(t.w); }
 
@@ -415,6 +568,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   __shared__ float s_red[NT / 32 + 1];
   const int tid = threadIdx.x;
   int wi = 0;
+#pragma unroll 1
   while (wi + 1 < S.n && (int)blockIdx.x >= S.w[wi + 1].cta0) ++wi;
   // the work and its propagator's descriptor in shared memory (the parameter
   // block is too large for the constant cache to keep)
@@ -424,22 +578,23 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     static_assert(sizeof(WaveWork) % 4 == 0 && sizeof(DevProp) % 4 == 0, "copied by words");
     const int* const a = reinterpret_cast<const int*>(&S.w[wi]);
     const int* const b = reinterpret_cast<const int*>(S.w[wi].prop);
+#pragma unroll 1
     for (int k = tid; k < (int)(sizeof(WaveWork) / 4); k += NT) reinterpret_cast<int*>(&w)[k] = a[k];
+#pragma unroll 1
     for (int k = tid; k < (int)(sizeof(DevProp) / 4); k += NT) reinterpret_cast<int*>(&P)[k] = b[k];
     __syncthreads();
   }
   const Geo G(P);
   const int nL = VISCO ? P.L : 0;
-  const int ng = (G.nxp + 3) / 4;
   const int cta = (int)blockIdx.x - w.cta0;
-  const WaveTile T = wave_tile(G.nzp, ng, w.pz, w.px, cta);
+  const WaveTile T = wave_tile(w.cut, w.pz, w.px, cta);
   const int i0 = T.i0, th = T.th, gw = T.gw, j0 = 4 * T.g0;
   int sx0, nsx, sz0, nsz;
   wave_strip(j0, min(j0 + 4 * gw, G.nxp), G.nxp, G.npx_l, G.npx_r, sx0, nsx);
   wave_strip(i0, i0 + th, G.nzp, G.npz_t, G.npz_b, sz0, nsz);
   const int ekind = w.epi.kind;
-  const int n_epi = (ekind == EPI_NONE) ? 0 : (EL && w.epi.need_s ? 2 : 1);
-  const WaveLayout Y = wave_layout(EL, VISCO, nL, RES, w.pad, th, gw, nsx, nsz, n_epi);
+  const int n_epi = (!EL || ekind == EPI_NONE) ? 0 : (w.epi.need_s ? 2 : 1);   // P and S kept beside the fields
+  const WaveLayout Y = wave_layout(EL, VISCO, nL, RES, w.pad, th, gw, nsx, nsz, n_epi, w.n_src, w.n_acc);
   const int W = Y.W, cw = Y.cw;
   float* const own = sm + Y.field + WAVE_HALO * W + WAVE_HALO;   // own cell (0, 0) of field 0
   const int FN = Y.field_n;
@@ -448,6 +603,8 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   unsigned char* const qsm = reinterpret_cast<unsigned char*>(sm + Y.qidx);
   float* const e_p = sm + Y.epi;
   float* const e_s = e_p + CN;
+  float* const e_src = sm + Y.src;
+  float* const accs = sm + Y.acc;
   const float4* const coltab = reinterpret_cast<const float4*>(sm + Y.col);
   const float4* const rowtab = reinterpret_cast<const float4*>(sm + Y.row);
   // ψ of x term t at (row r, strip column s): psx(t)[r·pxw + s]; of z term t
@@ -464,18 +621,16 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   // cell arrays (RES): acoustic dt·κ dt·irx dt·irz; elastic λ λ+2μ dt·μ dt·irx dt·irz;
   // viscoacoustic K_R dt·irx dt·irz b_l ε r_l
   const size_t fs = (size_t)(P.f[1] - P.f[0]);   // pitch of fields and coefficients
-  // interior CTA: every cell physical, clear of strips, free surface and source
-  const bool fast = i0 >= G.pad && i0 + th <= G.pad + G.nz && j0 >= G.pad && j0 + cw <= G.pad + G.nx && nsx == 0 &&
-                    nsz == 0 && (!G.free_surface || i0 > G.pad) &&
-                    !(G.src_iz >= i0 && G.src_iz < i0 + th && G.src_ix >= j0 && G.src_ix < j0 + cw);
-
   // ------------------------------------------------------------------ load
   if (tid == 0) s_abort = 0;
+#pragma unroll 1
   for (int k = tid; k < NF * FN / 4; k += NT) st4(sm + Y.field + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
   if (RES)
+#pragma unroll 1
     for (int k = tid; k < (Y.psix - Y.cell) / 4; k += NT) st4(sm + Y.cell + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
   __syncthreads();
   const ptrdiff_t ld_delta = w.load ? w.load - P.f[0] : 0;
+#pragma unroll 1
   for (int k = tid; k < th * gw; k += NT) {
     const int r = k / gw, c4 = 4 * (k - r * gw);
     const size_t g = (size_t)(i0 + r) * G.ld + j0 + c4;
@@ -497,7 +652,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         st4(cells + 0 * CN + o, ldg4(P.coef[CV_KR] + g));
         scaled(1, P.coef[CV_IRX]);
         scaled(2, P.coef[CV_IRZ]);
+#pragma unroll 1
         for (int l = 0; l < nL; ++l) st4(cells + (3 + l) * CN + o, ldg4(P.coef[CV_B0 + l] + g));
+#pragma unroll 1
         for (int l = 0; l <= nL; ++l) st4(cells + (3 + nL + l) * CN + o, ld4(P.f[V_EPS + l] + ld_delta + g));
         *reinterpret_cast<uchar4*>(qsm + o) = *reinterpret_cast<const uchar4*>(P.qidx + g);
       } else {
@@ -506,30 +663,35 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         scaled(2, P.coef[CA_IRZ]);
       }
     } else if (VISCO && ld_delta != 0) {
+#pragma unroll 1
       for (int l = 0; l <= nL; ++l) st4(P.f[V_EPS + l] + g, ld4(P.f[V_EPS + l] + ld_delta + g));
     }
   }
   if (RES || ld_delta != 0) {
 #pragma unroll
     for (int t = 0; t < NPSI; ++t) {
+#pragma unroll 1
       for (int k = tid; k < th * nsx; k += NT) {
         const int r = k / nsx, s = k - r * nsx;
         psx(t)[r * pxw + sx0 + s] = (P.psix[t] + ld_delta)[(size_t)(i0 + r) * G.wx + sx0 + s];
       }
+#pragma unroll 1
       for (int k = tid; k < nsz * gw; k += NT) {
         const int s = k / gw, c4 = 4 * (k - s * gw);
         st4(psz(t) + (sz0 + s) * pzw + c4, ld4(P.psiz[t] + ld_delta + (size_t)(sz0 + s) * G.ld + j0 + c4));
       }
     }
   }
+#pragma unroll 1
   for (int k = tid; k < cw; k += NT) {
     const int j = j0 + k, jc = min(j, G.nxp - 1), s = j < G.nxp ? G.sx(j) : -1;
-    const int f = (j >= M && j < G.nxp - M ? WAVE_IN : 0) | (j < G.nxp ? WAVE_OK : 0) | (j == G.src_ix ? WAVE_SRC : 0);
+    const int f = (j >= M && j < G.nxp - M ? WAVE_IN : 0) | (j < G.nxp ? WAVE_OK : 0);
     st4(sm + Y.col + 4 * k, make_float4(P.ax[jc], P.bx[jc], __int_as_float(s), __int_as_float(f)));
   }
+#pragma unroll 1
   for (int k = tid; k < th; k += NT) {
     const int i = i0 + k;
-    const int f = (i >= M && i < G.nzp - M ? WAVE_IN : 0) | (i == G.src_iz ? WAVE_SRC : 0) |
+    const int f = (i >= M && i < G.nzp - M ? WAVE_IN : 0) |
                   (G.free_surface && i == G.pad ? WAVE_SURFACE : 0);
     st4(sm + Y.row + 4 * k, make_float4(P.az[i], P.bz[i], __int_as_float(G.sz(i)), __int_as_float(f)));
   }
@@ -538,9 +700,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   const int nu = Y.units_n;
   {
     int4* const tab = reinterpret_cast<int4*>(sm + Y.units);
-    const int thmax = (G.nzp + w.pz - 1) / w.pz;   // the tallest CTA of the split
+#pragma unroll 1
     for (int k = tid; k < 2 * nu; k += NT) {
-      const WaveUnit q = wave_unit(EL, k / nu, k % nu, T, w.px, w.pz, thmax, W);
+      const WaveUnit q = wave_unit(EL, k / nu, k % nu, T, w.px, w.pz, w.thmax, W);
       const int64_t at = ((int64_t)blockIdx.x * 2 + k / nu) * S.half;
       const int64_t from = ((int64_t)(w.cta0 + q.nb) * 2 + k / nu) * S.half;
       tab[k] = make_int4(q.slot * FN + q.src, q.slot * FN + q.dst, (int)(at + q.put), q.nb < 0 ? -1 : (int)(from + q.get));
@@ -567,13 +729,14 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   float last_peak = 0.f;
   bool bad = false;
   const int mech = P.mech;
-  // the thread's cells: (row, first column) tid, tid + NT, … in row-major
-  // order of C-cell groups
+  // the thread's cells: blocks of C cells tid, tid + NT, … in row-major
+  // order; body(first row, first column)
   const int nv = cw / C;
   const int row0 = tid / nv, col0 = (tid - row0 * nv) * C;
   const int drow = NT / nv, dcol = (NT - drow * nv) * C;
   auto each = [&](auto&& body) {
     int r = row0, c = col0;
+#pragma unroll 1
     while (r < th) {
       body(r, c);
       r += drow;
@@ -585,6 +748,72 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     }
   };
 
+  // the CTA's straight-line rectangle; the frame around it takes the general
+  // form of the updates
+  const WaveInner I = wave_inner(G, T, C);
+  const int nb = I.nb, b0 = I.b0, b1 = I.b1, v0 = I.v0, v1 = I.v1;
+  const int n_inner = (b1 - b0) * (v1 - v0), n_frame = nb * nv - n_inner;
+  auto frame_block = [&](int k, int& r, int& c) {   // rows above, rows below, then the sides
+    const int above = b0 * nv, below = (nb - b1) * nv;
+    int b, v;
+    if (k < above) {
+      b = k / nv;
+      v = k - b * nv;
+    } else if (k < above + below) {
+      k -= above;
+      b = k / nv;
+      v = k - b * nv;
+      b += b1;
+    } else {
+      k -= above + below;
+      const int side = nv - (v1 - v0);
+      b = k / side;
+      v = k - b * side;
+      b += b0;
+      if (v >= v0) v += v1 - v0;
+    }
+    r = b;
+    c = v * C;
+  };
+  const int wi_ = max(v1 - v0, 1);
+  const int in_r = b0 + tid / wi_, in_c = (v0 + tid % wi_) * C;   // the thread's first inner block
+  const int in_dr = NT / wi_, in_dc = NT % wi_ * C;
+  int fr_r = 0, fr_c = 0;                                               // and its first frame block
+  if (tid < n_frame) frame_block(tid, fr_r, fr_c);
+  auto update = [&](auto&& body) {
+#pragma unroll 1
+    for (int k = tid, r = in_r, c = in_c; k < n_inner; k += NT) {
+      body(std::false_type{}, r, c);
+      r += in_dr;
+      c += in_dc;
+      if (c >= v1 * C) {
+        c -= (v1 - v0) * C;
+        ++r;
+      }
+    }
+#pragma unroll 1
+    for (int k = tid, r = fr_r, c = fr_c; k < n_frame;) {
+      body(std::true_type{}, r, c);
+      k += NT;
+      if (k < n_frame) frame_block(k, r, c);
+    }
+  };
+  // the source: its cell's owner adds the amplitude after its update
+  const bool src_here = w.wavelet && G.src_iz >= i0 && G.src_iz < i0 + th && G.src_ix >= j0 && G.src_ix < j0 + cw &&
+                        G.src_ix < G.nxp;
+  const int src_o = src_here ? (G.src_iz - i0) * W + G.src_ix - j0 : 0;
+  const int src_e = src_here ? (G.src_iz - i0) * cw + G.src_ix - j0 : 0;
+  int src_tid = -1;   // the thread that updates the source's block (frame_block and the inner walk inverted)
+  if (src_here) {
+    const int b = G.src_iz - i0, v = (G.src_ix - j0) / C, side = nv - (v1 - v0);
+    int k;
+    if (b >= b0 && b < b1 && v >= v0 && v < v1) k = (b - b0) * (v1 - v0) + v - v0;
+    else if (b < b0) k = b * nv + v;
+    else if (b >= b1) k = b0 * nv + (b - b1) * nv + v;
+    else k = (b0 + nb - b1) * nv + (b - b0) * side + (v < v0 ? v : v - (v1 - v0));
+    src_tid = k % NT;
+  }
+
   // injection: the thread's first cell and its first contribution
   auto inject_cell = [&](int q) -> float* {
     const int ij = w.inj.ij[q], s = w.inj.slot[q], i = ij >> 16, j = ij & 0xffff;
@@ -593,8 +822,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     return own + s * FN + (i - i0) * W + j - j0;
   };
   float* inj_cell = nullptr;
-  int inj_c0 = 0, inj_c1 = 0, inj_src = 0;
+  int inj_c0 = 0, inj_c1 = 0;
   double inj_wa = 0.0, inj_wb = 0.0;
+  const float* inj_p = w.inj.record;   // some valid address where there is no contribution
   float inj_v = 0.f;
   if (inj_a + tid < inj_b) {
     const int q = inj_a + tid;
@@ -602,26 +832,36 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     inj_c0 = w.inj.start[q];
     inj_c1 = w.inj.start[q + 1];
     if (inj_c0 < inj_c1) {
-      inj_src = w.inj.src[inj_c0];
+      inj_p += w.inj.src[inj_c0] + (int64_t)w.t0 * w.inj.nrec;
       inj_wa = w.inj.wa[inj_c0];
       inj_wb = w.inj.wb[inj_c0];
-      inj_v = w.inj.record[inj_src + (int64_t)w.t0 * w.inj.nrec];
+      inj_v = *inj_p;
     }
   }
 
+  // hot scalars of the work in registers (it lies in shared memory), and what
+  // this CTA does between steps: nothing for most CTAs of a forward run
+  const int n_steps = w.n_steps, sign = w.sign, flags = w.flags, n_acc = w.n_acc;
+  const bool between = ekind != EPI_NONE || smp_b > smp_a || inj_b > inj_a || n_acc;
+  const bool has_ck = w.ck != nullptr;
+  uint64_t* const xbuf = S.xbuf;
+  const int64_t plane = S.plane;
+
   // Publish this phase's edges; the caller may do other work, then collects.
   auto publish = [&](int ph, uint32_t e) {
+#pragma unroll 1
     for (int u = tid; u < nu; u += NT) {
       const int4 q = tab0[ph * nu + u];
-      if (q.w >= 0) wave_put(S.xbuf + 2 * (size_t)q.z, S.plane, ld4(own + q.x), e);
+      if (q.w >= 0) wave_put(xbuf + 2 * (size_t)q.z, plane, ld4(own + q.x), e);
     }
   };
   auto collect = [&](int ph, uint32_t e) {
+#pragma unroll 1
     for (int u = tid; u < nu; u += NT) {
       const int4 q = tab0[ph * nu + u];
       if (q.w < 0) continue;
       float4 v;
-      if (wave_get(S.xbuf + 2 * (size_t)q.w, S.plane, e, v)) st4(own + q.y, v);
+      if (wave_get(xbuf + 2 * (size_t)q.w, plane, e, v)) st4(own + q.y, v);
       else s_abort = 1;
     }
   };
@@ -631,23 +871,59 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     bool run = ekind != EPI_NONE && !((w.flags & WAVE_SKIP_LAST) && k + 1 == w.n_steps);
     if (t < w.start_step && (ekind == EPI_EXC_IMAGE || (ekind == EPI_IMAGE && !w.epi.illum && !w.epi.rillum)))
       run = false;
-    if (run) {
+    if (run && w.n_acc) cp_async_wait_all();   // each thread staged its own cells
+    if (run && !w.n_acc && ekind == EPI_IMAGE && !w.epi.kahan) {
+      // two blocks of the thread at a time (four spill registers)
+      constexpr int U = 2;
+      int r = row0, c0 = col0;
+#pragma unroll 1
+      while (r < th) {
+        WavePieces<U, C> K;
+        K.ok = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int ii = i0 + r - G.pad, jj = j0 + c0 - G.pad;
+          K.at[u] = (ptrdiff_t)ii * G.nx + jj;
+          if (r < th && ii >= 0 && ii < G.nz) {
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+              if (jj + c >= 0 && jj + c < G.nx) K.ok |= 1u << (u * C + c);
+            if constexpr (EL) ldv<C>(e_p + r * cw + c0, K.pv[u]);
+            else ldv<C>(own + A_P * FN + r * W + c0, K.pv[u]);
+            if (n_epi == 2) ldv<C>(e_s + r * cw + c0, K.sv[u]);
+          }
+          r += drow;
+          c0 += dcol;
+          if (c0 >= cw) {
+            c0 -= cw;
+            ++r;
+          }
+        }
+        wave_image_global<U, C>(w, t, K);
+      }
+    } else if (run) {
       each([&](int r, int c0) {
         const int ii = i0 + r - G.pad, jj = j0 + c0 - G.pad;
         if (ii < 0 || ii >= G.nz) return;
-        bool ok[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) ok[c] = jj + c >= 0 && jj + c < G.nx;
         float pv[C], sv[C] = {};
-        ldv<C>(e_p + r * cw + c0, pv);
+        if constexpr (EL) ldv<C>(e_p + r * cw + c0, pv);
+        else ldv<C>(own + A_P * FN + r * W + c0, pv);
         if (n_epi == 2) ldv<C>(e_s + r * cw + c0, sv);
-        wave_epilogue<C>(w, t, (ptrdiff_t)ii * G.nx + jj, ok, npix, pv, sv);
+        if (n_acc) {   // cells outside the physical grid sum into slots nobody reads
+          wave_image_resident<C>(w.epi, t >= w.start_step, accs, e_src, CN, r * cw + c0, pv, sv);
+        } else {
+          bool ok[C];
+#pragma unroll
+          for (int c = 0; c < C; ++c) ok[c] = jj + c >= 0 && jj + c < G.nx;
+          wave_epilogue<C>(w, t, (ptrdiff_t)ii * G.nx + jj, ok, npix, pv, sv);
+        }
       });
     }
     if (smp_off != -1) {
       // the thread's first corner cell; further ones from the list
       float* const row = w.smp.buf + (int64_t)k * w.smp.stride;
       row[smp_out] = smp_off >= 0 ? own[smp_off] : fmul(0.5f, fadd(own[E_SXX * FN - smp_off - 2], own[E_SZZ * FN - smp_off - 2]));
+#pragma unroll 1
       for (int q = smp_a + tid + NT; q < smp_b; q += NT) {
         const int ij = w.smp.ij[q], s = w.smp.slot[q];
         const int o = ((ij >> 16) - i0) * W + (ij & 0xffff) - j0;
@@ -655,8 +931,54 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
       }
     }
   };
+  // Stage the source fields of time t for finish(): each thread its own cells.
+  auto stage_sources = [&](int t) {
+    const ptrdiff_t s = (ptrdiff_t)(t - w.slot_t) * w.slot_floats;
+    each([&](int r, int c0) {
+      const int ii = i0 + r - G.pad, jj = j0 + c0 - G.pad;
+      if (ii < 0 || ii >= G.nz) return;
+      int n = 0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (!w.epi.src[k]) continue;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          if (jj + c >= 0 && jj + c < G.nx)
+            cp_async4(e_src + n * CN + r * cw + c0 + c, w.epi.src[k] + s + (ptrdiff_t)ii * G.nx + jj + c);
+        ++n;
+      }
+    });
+    cp_async_commit();
+  };
+  // Imaging sums between global memory and their resident copies.
+  auto move_sums = [&](bool in) {
+#pragma unroll 1
+    for (int k = tid; k < th * cw; k += NT) {
+      const int r = k / cw, c = k - r * cw, ii = i0 + r - G.pad, jj = j0 + c - G.pad;
+      if (ii < 0 || ii >= G.nz || jj < 0 || jj >= G.nx) continue;
+      const size_t p = (size_t)ii * G.nx + jj;
+      wave_each_sum(w.epi, [&](int q, double* g) {
+        float* const a = accs + 2 * q * CN;
+        if (!w.epi.kahan) {
+          double* const d = reinterpret_cast<double*>(a) + k;
+          if (in) *d = g[p];
+          else g[p] = *d;
+        } else {
+          float* const f = reinterpret_cast<float*>(g);
+          if (in) {
+            a[k] = f[p];
+            a[CN + k] = f[npix + p];
+          } else {
+            f[p] = a[k];
+            f[npix + p] = a[CN + k];
+          }
+        }
+      });
+    }
+  };
   // Write the CTA's part of the state into a state block (own or checkpoint).
   auto store_state = [&](ptrdiff_t delta) {
+#pragma unroll 1
     for (int k = tid; k < th * gw; k += NT) {
       const int r = k / gw, c4 = 4 * (k - r * gw);
       const size_t g = (size_t)(i0 + r) * G.ld + j0 + c4;
@@ -664,6 +986,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
       for (int f = 0; f < NF; ++f) st4(P.f[f] + delta + g, ld4(own + f * FN + r * W + c4));
       if constexpr (VISCO) {
         if (RES || delta != 0)
+#pragma unroll 1
           for (int l = 0; l <= nL; ++l)
             st4(P.f[V_EPS + l] + delta + g,
                 RES ? ld4(cells + (3 + nL + l) * CN + r * cw + c4) : ld4(P.f[V_EPS + l] + g));
@@ -672,10 +995,12 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     if (RES || delta != 0) {
 #pragma unroll
       for (int t = 0; t < NPSI; ++t) {
+#pragma unroll 1
         for (int k = tid; k < th * nsx; k += NT) {
           const int r = k / nsx, s = k - r * nsx;
           (P.psix[t] + delta)[(size_t)(i0 + r) * G.wx + sx0 + s] = psx(t)[r * pxw + sx0 + s];
         }
+#pragma unroll 1
         for (int k = tid; k < nsz * gw; k += NT) {
           const int s = k / gw, c4 = 4 * (k - s * gw);
           st4(P.psiz[t] + delta + (size_t)(sz0 + s) * G.ld + j0 + c4, ld4(psz(t) + (sz0 + s) * pzw + c4));
@@ -735,35 +1060,69 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     }
   };
 
+  // pressure engines image p itself, so a CTA that injects finishes a step
+  // before the next one's injection, every other CTA after publishing
+  const bool early = !EL && inj_b > inj_a;
+  int t = w.t0;
+  uint32_t e = w.epoch + 1;
 #pragma unroll 1
-  for (int k = 0; k < w.n_steps; ++k) {
-    const int t = w.t0 + w.sign * k;
-    const uint32_t e = w.epoch + 1 + 2 * (uint32_t)k;
-    // ------------------------------------------------------------- injection
-    if (inj_b > inj_a) {
-      const int64_t off = (int64_t)t * w.inj.nrec;
-      for (int q = inj_a + tid; q < inj_b; q += NT) {
-        const bool mine = q == inj_a + tid;   // the thread's first cell: its list entry is in registers
-        const int c1 = mine ? inj_c1 : w.inj.start[q + 1];
-        int c = mine ? inj_c0 : w.inj.start[q];
-        float* f = mine ? inj_cell : inject_cell(q);
-        float acc = *f;
-        if (mine && c < c1) {
-          acc = __double2float_rn(dadd((double)acc, dmul(dmul((double)inj_v, inj_wa), inj_wb)));
-          ++c;
+  for (int k = 0;; ++k, t += sign, e += 2) {
+    if (between) {
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {   // one copy of finish()
+        if (k > 0 && (pass == 0) == early) {
+          finish(k - 1);
+          if (early) __syncthreads();
         }
-        for (; c < c1; ++c) {
-          const double v = (double)w.inj.record[w.inj.src[c] + off];
-          acc = __double2float_rn(dadd((double)acc, dmul(dmul(v, w.inj.wa[c]), w.inj.wb[c])));
+        if (pass == 0 && k < n_steps) {
+          if (inj_b > inj_a) {
+            const int64_t off = (int64_t)t * w.inj.nrec;
+#pragma unroll 1
+            for (int q = inj_a + tid; q < inj_b; q += NT) {
+              const bool mine = q == inj_a + tid;   // the thread's first cell: its list entry is in registers
+              const int c1 = mine ? inj_c1 : w.inj.start[q + 1];
+              int c = mine ? inj_c0 : w.inj.start[q];
+              float* f = mine ? inj_cell : inject_cell(q);
+              float acc = *f;
+              if (mine && c < c1) {
+                acc = __double2float_rn(dadd((double)acc, dmul(dmul((double)inj_v, inj_wa), inj_wb)));
+                ++c;
+              }
+#pragma unroll 1
+              for (; c < c1; ++c) {
+                const double v = (double)w.inj.record[w.inj.src[c] + off];
+                acc = __double2float_rn(dadd((double)acc, dmul(dmul(v, w.inj.wa[c]), w.inj.wb[c])));
+              }
+              *f = acc;
+            }
+            __syncthreads();
+            // the next step's sample of the first contribution, in flight until then
+            if (k + 1 < n_steps) inj_p += sign * w.inj.nrec;
+            inj_v = *inj_p;
+          }
+          publish(0, e);
         }
-        *f = acc;
       }
-      __syncthreads();
-      // the next step's sample of the first contribution, in flight until then
-      if (inj_c0 < inj_c1 && k + 1 < w.n_steps) inj_v = w.inj.record[inj_src + off + w.sign * w.inj.nrec];
+      // the sums come in before the first step's imaging and go out after the
+      // last's
+      if (n_acc && (k == 0 || k == n_steps)) {
+        __syncthreads();
+        move_sums(k == 0);
+        __syncthreads();
+      }
+    } else if (k < n_steps) {
+      publish(0, e);
     }
-    publish(0, e);
-    if (k > 0) finish(k - 1);
+    if (k > 0 && (has_ck || k == n_steps)) {   // states go out after their step
+#pragma unroll 1
+      for (int out = 0; out < 2; ++out) {
+        const int done = t - sign;   // time of the last finished step
+        if (out == 0 ? (has_ck && done % w.ck_every == 0) : k == n_steps)
+          store_state(out == 0 ? (w.ck - P.f[0]) + (ptrdiff_t)(done / w.ck_every) * w.ck_floats : 0);
+      }
+    }
+    if (k == n_steps) break;
+    if (n_acc) stage_sources(t);
     collect(0, e);
     __syncthreads();
     if (s_abort) break;
@@ -772,41 +1131,41 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     auto velocity = [&](auto edge, int r, int c0) {
       constexpr bool EDGE = decltype(edge)::value;
       float* const at = own + r * W + c0;
-      float4 ct[C], rt;
+      float4 ct[C];
       if constexpr (EDGE) {
-        rt = rowtab[r];
 #pragma unroll
         for (int c = 0; c < C; ++c) ct[c] = coltab[c0 + c];
       }
+      float z1[C][9], z2[EL ? C : 1][9];
+      zwin<C>(at + (EL ? E_SXZ : A_P) * FN, W, z1);
+      if constexpr (EL) zwin<C>(at + E_SZZ * FN, W, z2);
+      float4 rt;
+      if constexpr (EDGE) rt = rowtab[r];
       const bool zin = !EDGE || (wave_flags_of(rt) & WAVE_IN);
       float ax[C], az[C], bx[C], bz[C];   // x and z terms of vx, then of vz
+      float v[8 + C];
       if constexpr (!EL) {
-        float v[8 + C], z[C][9];
         xwin<C>(at + A_P * FN, v);
-        zwin<C>(at + A_P * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           ax[c] = xin ? G.dxf(wave_plus(v, 4 + c)) : 0.f;
-          bz[c] = zin ? G.dzf(wave_plus(z[c], 4)) : 0.f;
+          bz[c] = zin ? G.dzf(wave_plus(z1[c], 4)) : 0.f;
         }
       } else {
-        float v[8 + C], z[C][9];
         xwin<C>(at + E_SXX * FN, v);
-        zwin<C>(at + E_SXZ * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           ax[c] = xin ? G.dxf(wave_plus(v, 4 + c)) : 0.f;
-          az[c] = zin ? G.dzf(wave_minus(z[c], 4)) : 0.f;
+          az[c] = zin ? G.dzf(wave_minus(z1[c], 4)) : 0.f;
         }
         xwin<C>(at + E_SXZ * FN, v);
-        zwin<C>(at + E_SZZ * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           bx[c] = xin ? G.dxf(wave_minus(v, 4 + c)) : 0.f;
-          bz[c] = zin ? G.dzf(wave_plus(z[c], 4)) : 0.f;
+          bz[c] = zin ? G.dzf(wave_plus(z2[c], 4)) : 0.f;
         }
       }
       if constexpr (EDGE) {
@@ -838,14 +1197,13 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
       stv<C>(pvx, ox);
       stv<C>(pvz, oz);
     };
-    if (fast) each([&](int r, int c0) { velocity(std::false_type{}, r, c0); });
-    else each([&](int r, int c0) { velocity(std::true_type{}, r, c0); });
+    update(velocity);
     __syncthreads();
     publish(1, e + 1);
     float amp = 0.f, amp_eps = 0.f;
-    if (!fast && w.wavelet) {
+    if (src_here) {
       amp = w.wavelet[t];
-      if (VISCO && amp != 0.f && G.src_iz >= 0)
+      if (VISCO && amp != 0.f)
         amp_eps = __double2float_rn(
             __ddiv_rn((double)amp, (double)P.coef[CV_KR][(size_t)G.src_iz * G.ld + G.src_ix]));
     }
@@ -857,28 +1215,29 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     auto stress = [&](auto edge, int r, int c0) {
       constexpr bool EDGE = decltype(edge)::value;
       float* const at = own + r * W + c0;
+      float z1[C][9], z2[EL ? C : 1][9];
+      zwin<C>(at + (EL ? E_VZ : A_VZ) * FN, W, z1);
+      if constexpr (EL) zwin<C>(at + E_VX * FN, W, z2);
       float4 ct[C], rt;
-      bool live[C], src[C];   // column of the grid; the source's cell (with a non-zero amplitude)
+      bool live[C];   // column of the grid
       if constexpr (EDGE) rt = rowtab[r];
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         if constexpr (EDGE) ct[c] = coltab[c0 + c];
         live[c] = !EDGE || (wave_flags_of(ct[c]) & WAVE_OK);
-        src[c] = EDGE && amp != 0.f && (wave_flags_of(ct[c]) & wave_flags_of(rt) & WAVE_SRC);
       }
       const bool zin = !EDGE || (wave_flags_of(rt) & WAVE_IN);
       const bool zstrip = EDGE && nsz && wave_strip_of(rt) >= 0;
       const bool surface = EDGE && (wave_flags_of(rt) & WAVE_SURFACE);
       float dx[C], dz[C];
       if constexpr (!EL) {
-        float v[8 + C], z[C][9];
+        float v[8 + C];
         xwin<C>(at + A_VX * FN, v);
-        zwin<C>(at + A_VZ * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           dx[c] = xin ? G.dxf(wave_minus(v, 4 + c)) : 0.f;
-          dz[c] = zin ? G.dzf(wave_minus(z[c], 4)) : 0.f;
+          dz[c] = zin ? G.dzf(wave_minus(z1[c], 4)) : 0.f;
         }
         if constexpr (EDGE) {
           float(*const ex[1])[C] = {&dx};
@@ -895,7 +1254,6 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
           for (int c = 0; c < C; ++c) {
             if (!live[c]) continue;
             out[c] = fadd(out[c], fmul(kk[c], fadd(dx[c], dz[c])));
-            if (src[c]) out[c] = fadd(out[c], amp);
             if (surface) out[c] = 0.f;
           }
         } else {
@@ -941,10 +1299,6 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
             if (!live[c]) continue;
             float ee = fadd(ev[c], inc[c]);
             float pv = fadd(fmul(kk[c], ee), tot[c]);
-            if (src[c]) {
-              ee = fadd(ee, amp_eps);
-              pv = fadd(pv, amp);
-            }
             ev[c] = ee;
             out[c] = pv;
             peak = fmaxf(peak, fabsf(pv));
@@ -954,27 +1308,24 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         stv<C>(pp, out);
 #pragma unroll
         for (int c = 0; c < C; ++c) bad |= nonfinite(out[c]);
-        if (n_epi) stv<C>(e_p + r * cw + c0, out);
       } else {
         float gx[C], gz[C], pv[C], sv[C] = {};   // ∂x vz and ∂z vx of σxz; P and S of the epilogue
-        float v[8 + C], z[C][9];
+        float v[8 + C];
         xwin<C>(at + E_VX * FN, v);
-        zwin<C>(at + E_VZ * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           dx[c] = xin ? G.dxf(wave_minus(v, 4 + c)) : 0.f;
-          dz[c] = zin ? G.dzf(wave_minus(z[c], 4)) : 0.f;
+          dz[c] = zin ? G.dzf(wave_minus(z1[c], 4)) : 0.f;
           pv[c] = fadd(dx[c], dz[c]);
         }
         xwin<C>(at + E_VZ * FN, v);
-        zwin<C>(at + E_VX * FN, W, z);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const bool xin = !EDGE || (wave_flags_of(ct[c]) & WAVE_IN);
           gx[c] = xin ? G.dxf(wave_plus(v, 4 + c)) : 0.f;
-          gz[c] = zin ? G.dzf(wave_plus(z[c], 4)) : 0.f;
-          if (want_curl) sv[c] = fsub(G.dzf(wave_minus(z[c], 4)), G.dxf(wave_minus(v, 4 + c)));
+          gz[c] = zin ? G.dzf(wave_plus(z2[c], 4)) : 0.f;
+          if (want_curl) sv[c] = fsub(G.dzf(wave_minus(z2[c], 4)), G.dxf(wave_minus(v, 4 + c)));
         }
         if constexpr (EDGE) {
           float(*const ex[2])[C] = {&dx, &gx};
@@ -998,14 +1349,6 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
           oxx[c] = fadd(oxx[c], fmul(G.dt, fadd(fmul(l2m[c], dx[c]), fmul(lam[c], dz[c]))));
           ozz[c] = fadd(ozz[c], fmul(G.dt, fadd(fmul(lam[c], dx[c]), fmul(l2m[c], dz[c]))));
           oxz[c] = fadd(oxz[c], fmul(dmu[c], fadd(gz[c], gx[c])));
-          if (src[c]) {
-            if (mech == MECH_SHEAR) {
-              oxz[c] = fadd(oxz[c], amp);
-            } else if (mech == MECH_EXPLOSIVE) {
-              oxx[c] = fadd(oxx[c], amp);
-              ozz[c] = fadd(ozz[c], amp);
-            }
-          }
           if (surface) {
             ozz[c] = 0.f;
             oxz[c] = 0.f;
@@ -1029,34 +1372,61 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         }
       }
     };
-    if (fast) each([&](int r, int c0) { stress(std::false_type{}, r, c0); });
-    else each([&](int r, int c0) { stress(std::true_type{}, r, c0); });
-    __syncthreads();
-    // a vertical force lands on vz after the stress phase
-    if (EL && mech == MECH_FORCE_Z && amp != 0.f && tid == 0 && G.src_iz >= i0 && G.src_iz < i0 + th &&
-        G.src_ix >= j0 && G.src_ix < j0 + cw) {
-      float* const f = own + E_VZ * FN + (G.src_iz - i0) * W + G.src_ix - j0;
-      *f = fadd(*f, amp);
+    update(stress);
+    // the source, by the thread that has just updated its cell
+    if (tid == src_tid && amp != 0.f) {
+      auto add = [&](float* f, float a) {
+        *f = fadd(*f, a);
+        bad |= nonfinite(*f);
+      };
+      const bool surface = G.free_surface && G.src_iz == G.pad;   // the surface zeroes p, σzz and σxz after it
+      if constexpr (EL) {
+        if (mech == MECH_SHEAR) {
+          if (!surface) add(own + E_SXZ * FN + src_o, amp);
+        } else if (mech == MECH_EXPLOSIVE) {
+          add(own + E_SXX * FN + src_o, amp);
+          if (!surface) add(own + E_SZZ * FN + src_o, amp);
+        }
+        if (n_epi && esep == 0) {
+          e_p[src_e] = fmul(0.5f, fadd(own[E_SXX * FN + src_o], own[E_SZZ * FN + src_o]));
+          if (n_epi == 2) e_s[src_e] = own[E_SXZ * FN + src_o];
+        }
+      } else if (!surface) {
+        add(own + A_P * FN + src_o, amp);
+        if constexpr (VISCO) {
+          const size_t g = (size_t)G.src_iz * G.ld + G.src_ix;
+          add(RES ? cells + (3 + nL) * CN + src_e : P.f[V_EPS] + g, amp_eps);
+        }
+      }
     }
-    if (EL && mech == MECH_FORCE_Z && amp != 0.f) __syncthreads();
+    __syncthreads();
+    if (EL && mech == MECH_FORCE_Z && src_here && amp != 0.f) {
+      // a vertical force lands on vz once every thread has read it
+      if (tid == src_tid) own[E_VZ * FN + src_o] = fadd(own[E_VZ * FN + src_o], amp);
+      __syncthreads();
+    }
     // -------------------------------------------- compensated amplitude cap
-    if (VISCO && (w.flags & WAVE_STAB)) {
+    if (VISCO && (flags & WAVE_STAB)) {
       const int ncta = w.px * w.pz;
+#pragma unroll 1
       for (int o = 16; o > 0; o >>= 1) peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, o));
       if ((tid & 31) == 0) s_red[tid >> 5] = peak;
       __syncthreads();
       uint64_t* const words = S.peaks + (size_t)(k & 1) * gridDim.x + w.cta0;
       if (tid == 0) {
         float m = s_red[0];
+#pragma unroll 1
         for (int q = 1; q < NT / 32; ++q) m = fmaxf(m, s_red[q]);
         const uint64_t word = ((uint64_t)e << 32) | __float_as_uint(m);
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(words + cta), "l"(word) : "memory");
       }
       __syncthreads();
       float m = 0.f;
+#pragma unroll 1
       for (int q = tid; q < ncta; q += NT) {
         uint64_t word = 0;
         int it = 0;
+#pragma unroll 1
         for (; it < WAVE_SPIN_LIMIT; ++it) {
           asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(word) : "l"(words + q) : "memory");
           if ((uint32_t)(word >> 32) == e) break;
@@ -1064,11 +1434,13 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         if (it == WAVE_SPIN_LIMIT) s_abort = 1;
         m = fmaxf(m, __uint_as_float((uint32_t)word));
       }
+#pragma unroll 1
       for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       if ((tid & 31) == 0) s_red[tid >> 5] = m;
       __syncthreads();
       if (s_abort) break;
       m = s_red[0];
+#pragma unroll 1
       for (int q = 1; q < NT / 32; ++q) m = fmaxf(m, s_red[q]);
       last_peak = m;
       const double pk = (double)m;
@@ -1083,21 +1455,22 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
             const float4 v = ld4(f);
             st4(f, make_float4(fmul(v.x, s), fmul(v.y, s), fmul(v.z, s), fmul(v.w, s)));
           };
+#pragma unroll 1
           for (int q = tid; q < th * gw; q += NT) {
             const int r = q / gw, c4 = 4 * (q - r * gw);
 #pragma unroll
             for (int f = 0; f < NF; ++f) scale4(own + f * FN + r * W + c4);
             const size_t g = (size_t)(i0 + r) * G.ld + j0 + c4;
+#pragma unroll 1
             for (int l = 0; l <= nL; ++l)
               scale4(RES ? cells + (3 + nL + l) * CN + r * cw + c4 : P.f[V_EPS + l] + g);
-            if (n_epi) scale4(e_p + r * cw + c4);
           }
         }
       }
       __syncthreads();
     }
-    if (w.ck && t % w.ck_every == 0) store_state((w.ck - P.f[0]) + (ptrdiff_t)(t / w.ck_every) * w.ck_floats);
   }
+  cp_async_wait_all();   // never leave with copies into shared memory in flight
   __syncthreads();
   if (bad) atomicOr(P.status, STATUS_NONFINITE);
   if (s_abort) {
@@ -1105,8 +1478,6 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     return;
   }
   if (w.n_steps > 0) {
-    finish(w.n_steps - 1);
-    store_state(0);
     if (VISCO && (w.flags & WAVE_STAB) && cta == 0 && tid == 0) {
       w.stab->ref_amp = ref_amp;
       w.stab->clipped += clipped;
