@@ -824,7 +824,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   float* inj_cell = nullptr;
   int inj_c0 = 0, inj_c1 = 0;
   double inj_wa = 0.0, inj_wb = 0.0;
-  const float* inj_p = w.inj.record;   // some valid address where there is no contribution
+  // (threads without a contribution follow the record's rows at column 0, so
+  // the look-ahead below is an unconditional load inside the record)
+  const float* inj_p = w.inj.cta ? w.inj.record + (int64_t)w.t0 * w.inj.nrec : nullptr;
   float inj_v = 0.f;
   if (inj_a + tid < inj_b) {
     const int q = inj_a + tid;
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     inj_c0 = w.inj.start[q];
     inj_c1 = w.inj.start[q + 1];
     if (inj_c0 < inj_c1) {
-      inj_p += w.inj.src[inj_c0] + (int64_t)w.t0 * w.inj.nrec;
+      inj_p += w.inj.src[inj_c0];
       inj_wa = w.inj.wa[inj_c0];
       inj_wb = w.inj.wb[inj_c0];
       inj_v = *inj_p;
