@@ -461,10 +461,10 @@ __device__ __forceinline__ void run_epilogue(const Epilogue& E, size_t c, size_t
 // accumulator, replay and excitation accesses coalesce whatever their
 // alignment.  One copy of the epilogue code serves every cell.
 //
-// The imaging condition gathers: a thread loads the replayed source values of
-// all its cells, then, accumulator by accumulator, loads all its cells' sums
-// (float64, or Kahan float32 sum and compensation) before it adds and stores
-// them, so several global loads are in flight per thread instead of one.
+// The imaging condition with float64 sums (the common case) gathers: a thread
+// loads the replayed source values of all its cells, then, accumulator by
+// accumulator, loads all its cells' sums before it adds and stores them, so
+// several global loads are in flight per thread instead of one.
 template <int IT>
 struct ImageCells {
   uint32_t pc[IT];
@@ -482,28 +482,9 @@ __device__ __forceinline__ void accumulate_cells(double* acc, const ImageCells<I
     if (C.ok[it]) acc[C.pc[it]] = dadd(a[it], (double)term(it));
 }
 
-template <int IT, class TERM>
-__device__ __forceinline__ void accumulate_cells_kahan(double* acc, size_t npix, const ImageCells<IT>& C, TERM term) {
-  float* const sum = reinterpret_cast<float*>(acc);
-  float* const cmp = sum + npix;
-  float a[IT], k[IT];
-#pragma unroll
-  for (int it = 0; it < IT; ++it) {
-    a[it] = C.ok[it] ? sum[C.pc[it]] : 0.f;
-    k[it] = C.ok[it] ? cmp[C.pc[it]] : 0.f;
-  }
-#pragma unroll
-  for (int it = 0; it < IT; ++it)
-    if (C.ok[it]) {   // acc_term's update
-      const float y = fsub(term(it), k[it]), t = fadd(a[it], y);
-      cmp[C.pc[it]] = fsub(fsub(t, a[it]), y);
-      sum[C.pc[it]] = t;
-    }
-}
-
-template <int TZ, int NT, bool KAHAN, class GEO>
-__device__ __forceinline__ void image_tile(const Epilogue& E, const GEO& G, int i0, int j0, const float* e_p,
-                                           const float* e_s, size_t npix) {
+template <int TZ, int NT, class GEO>
+__device__ __forceinline__ void image_tile_f64(const Epilogue& E, const GEO& G, int i0, int j0, const float* e_p,
+                                               const float* e_s) {
   constexpr int IT = TZ * 32 / NT;
   const int tid = threadIdx.y * XT + threadIdx.x;
   ImageCells<IT> C;
@@ -526,13 +507,9 @@ __device__ __forceinline__ void image_tile(const Epilogue& E, const GEO& G, int 
     auto src = [&](int it) { return s_is_1 ? C.s1[it] : C.s0[it]; };
     auto rcv = [&](int it) { return r_is_s ? (e_s ? e_s[tid + it * NT] : 0.f) : e_p[tid + it * NT]; };
     // imaging.py:313-324: illum += S², rillum += R² (all steps); num += S·R (t ≥ start)
-    auto add = [&](double* acc, auto term) {
-      if constexpr (KAHAN) accumulate_cells_kahan(acc, npix, C, term);
-      else accumulate_cells(acc, C, term);
-    };
-    if (E.illum && E.ill[k]) add(E.ill[k], [&](int it) { return fmul(src(it), src(it)); });
-    if (E.rillum && E.ril[k]) add(E.ril[k], [&](int it) { return fmul(rcv(it), rcv(it)); });
-    if (E.cross) add(E.num[k], [&](int it) { return fmul(src(it), rcv(it)); });
+    if (E.illum && E.ill[k]) accumulate_cells(E.ill[k], C, [&](int it) { return fmul(src(it), src(it)); });
+    if (E.rillum && E.ril[k]) accumulate_cells(E.ril[k], C, [&](int it) { return fmul(rcv(it), rcv(it)); });
+    if (E.cross) accumulate_cells(E.num[k], C, [&](int it) { return fmul(src(it), rcv(it)); });
   }
 }
 
@@ -575,9 +552,8 @@ __device__ __forceinline__ void prefetch_image_tile(const Epilogue& E, const GEO
 template <int TZ, int NT, class GEO>
 __device__ __forceinline__ void epilogue_tile(const Epilogue& E, const GEO& G, int i0, int j0, const float* e_p,
                                               const float* e_s, size_t npix) {
-  if (E.kind == EPI_IMAGE && (TZ * 32) % NT == 0) {
-    if (E.kahan) image_tile<TZ, NT, true>(E, G, i0, j0, e_p, e_s, npix);
-    else image_tile<TZ, NT, false>(E, G, i0, j0, e_p, e_s, npix);
+  if (E.kind == EPI_IMAGE && !E.kahan && (TZ * 32) % NT == 0) {
+    image_tile_f64<TZ, NT>(E, G, i0, j0, e_p, e_s);
     return;
   }
   const int tid = threadIdx.y * XT + threadIdx.x;
