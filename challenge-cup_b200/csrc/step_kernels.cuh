@@ -417,14 +417,37 @@ __device__ __forceinline__ void run_epilogue(const Epilogue& E, size_t c, size_t
         }
         break;
       }
+      // Kahan sums: likewise every sum and compensation first, then acc_term's
+      // update of each
+      float a[3][MAX_EPI_IMAGES], q[3][MAX_EPI_IMAGES];
+      auto sum_of = [&](int kind, int k) -> float* {   // S², R², S·R
+        return reinterpret_cast<float*>(kind == 0 ? (E.illum ? E.ill[k] : nullptr)
+                                                  : (kind == 1 ? (E.rillum ? E.ril[k] : nullptr)
+                                                               : (E.cross ? E.num[k] : nullptr)));
+      };
+#pragma unroll
+      for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
+        if (k >= E.n_images) break;
+#pragma unroll
+        for (int kind = 0; kind < 3; ++kind)
+          if (const float* p = sum_of(kind, k)) {
+            a[kind][k] = p[c];
+            q[kind][k] = p[npix + c];
+          }
+      }
 #pragma unroll
       for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
         if (k >= E.n_images) break;
         const float s = E.src_slot[k] ? s1 : s0;
         const float r = E.rcv_wave[k] ? sv : pv;
-        if (E.illum && E.ill[k]) acc_term(E.ill[k], E.kahan, c, npix, fmul(s, s));
-        if (E.rillum && E.ril[k]) acc_term(E.ril[k], E.kahan, c, npix, fmul(r, r));
-        if (E.cross) acc_term(E.num[k], E.kahan, c, npix, fmul(s, r));
+#pragma unroll
+        for (int kind = 0; kind < 3; ++kind)
+          if (float* p = sum_of(kind, k)) {
+            const float term = kind == 0 ? fmul(s, s) : (kind == 1 ? fmul(r, r) : fmul(s, r));
+            const float y = fsub(term, q[kind][k]), t = fadd(a[kind][k], y);
+            p[npix + c] = fsub(fsub(t, a[kind][k]), y);
+            p[c] = t;
+          }
       }
       break;
     }
@@ -1088,6 +1111,12 @@ __device__ __forceinline__ void block_max_to(float v, float* dst) {
 template <bool VISCO, int KIND, int R>
 constexpr int kStressMinBlocks = (VISCO && KIND == TILES_INTERIOR && R == 1) ? 9 : 1;
 
+// Resident blocks per SM the elastic stress kernels are compiled for (0: the
+// compiler's own choice): the 32-row frame kernel takes 160 registers uncapped
+// (3 blocks), 128 capped for 4.
+template <int KIND, int R>
+constexpr int kElasticMinBlocks = (KIND == TILES_FRAME && R == 2) ? 4 : 0;
+
 // Acoustic (VISCO=false): p += (dt·κ)·div.  Viscoacoustic (VISCO=true):
 // ε += dt·div; r_l ← r_l·a_l + b_l·Δε; p = K_R·ε + Σ r_l.
 template <int M, int BZ, int R, bool VISCO, int KIND, class WS, class TM>
@@ -1284,7 +1313,7 @@ k_pressure_stress(const DevProp* __restrict__ props, const WS ws, const __grid_c
 // then the epilogue with P/S from the stresses (stress separation) or from
 // the raw velocity divergence/curl (divcurl, propagation.py:953-976).
 template <int M, int BZ, int R, int KIND, class WS, class TM>
-__global__ void __launch_bounds__(XT* BZ)
+__global__ void __launch_bounds__(XT* BZ, kElasticMinBlocks<KIND, R>)
 k_elastic_stress(const DevProp* __restrict__ props, const WS ws, const __grid_constant__ TM tm) {
   constexpr int TZ = BZ * R;
   using T = TileShape<M, TZ>;
