@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1422,6 +1423,14 @@ void launch_epilogue(Prop& P, const Epilogue& E) {
   ++g_launches;
 }
 
+// A shot's splits and its position in the multi-step schedule.
+struct WaveShot {
+  WavePlan whole, alone;   // the forward pass; a replay on every SM
+  WavePlan f, b;           // replay and backward, side by side where both fit
+  bool on = false, together = false;
+  int rb = -1, rt = 0, bb = -1, bt = 0;   // replay block and time, backward block and time
+};
+
 // Per-shot state of one migration: device buffers, epilogue template and
 // the position in the schedule (used by the plain and the batched drivers).
 struct ShotRun {
@@ -1437,7 +1446,7 @@ struct ShotRun {
   bool need_src[2] = {false, false}, need_rcv_s = false;
   bool bwd_unfused = false, fwd_unfused = false;
   int n_src = 1;               // source image fields stored per replayed step (P and/or S)
-  DevBuf wave, rec, acc, ck, rbuf[2], running, peak;
+  DevBuf wave_dev, rec, acc, ck, rbuf[2], running, peak;   // wave_dev: the wavelet
   std::vector<int64_t> ck_step;
   InjectPlanHost* plan = nullptr;
   double* num[MAX_EPI_IMAGES] = {};
@@ -1448,6 +1457,7 @@ struct ShotRun {
   // schedule: 0 forward, 1 replay/backward, 2 excitation map, 3 excitation backward, 4 done
   int phase = 0;
   int t_f = 0, rp_block = -1, rp_t = 0, bk_block = -1, bk_t = 0, replayed_below = 0;
+  WaveShot wave;
   int s_of(int b) const { return b * iv; }
   int e_of(int b) const { return std::min((b + 1) * iv, nt); }
 };
@@ -1497,8 +1507,8 @@ void prepare_run(ShotRun& R, Prop& F, Prop& B, const ertm_migrate_config& cfg, c
     R.num[k] = R.acc.as<double>() + k * npix;
     R.ril[k] = R.acc.as<double>() + (nimg + k) * npix;
   }
-  R.wave = DevBuf((size_t)R.nt * 4, st);
-  upload(R.wave.p, wavelet, (size_t)R.nt * 4, st);
+  R.wave_dev = DevBuf((size_t)R.nt * 4, st);
+  upload(R.wave_dev.p, wavelet, (size_t)R.nt * 4, st);
   std::vector<int> comps(cfg.comp, cfg.comp + cfg.n_comp);
   R.nrec = (int64_t)B.rx.size();
   R.rec = DevBuf((size_t)cfg.n_comp * cfg.nt_spec * R.nrec * 4, st);
@@ -1649,8 +1659,9 @@ void require_finite(const ShotRun& R, cudaStream_t st, const std::string& what) 
 // --------------------------------------------------------------------------
 // Multi-step launches (wave_kernel.cuh)
 // --------------------------------------------------------------------------
-// 0: where they are expected to be faster; 1: never; 2: wherever they fit.
-std::atomic<int> g_wave{0};
+// For the calling thread's calls: 0 where they are expected to be faster;
+// 1 never; 2 wherever they fit.
+thread_local int t_wave = 0;
 constexpr int kWaveSmemMax = 227 * 1024 - 2048;   // dynamic shared memory (the static part left out)
 constexpr int kWaveMaxSteps = 1024;               // steps per launch: keeps a launch to a few ms
 
@@ -1957,7 +1968,7 @@ WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& co
 // Grids the multi-step launches are used for: whatever fits with the
 // coefficients resident.
 bool wave_wanted(const WavePlan& p) {
-  const int mode = g_wave.load();
+  const int mode = t_wave;
   return p.ok() && mode != 1 && (mode == 2 || p.res);
 }
 
@@ -2004,16 +2015,9 @@ bool forward_wave(Prop& P, int nt, const float* dwave, const SampleSet& S, const
   return true;
 }
 
-// One shot through multi-step launches: the forward pass with checkpoints
-// written by the launches themselves, then, block by block, the replay of
-// block b − 1 beside the backward pass over block b (two works of one
-// launch, two replay buffers).  False when the shot does not qualify.
-struct WaveShot {
-  WavePlan whole, alone;   // the forward pass; a replay on every SM
-  WavePlan f, b;           // replay and backward, side by side where both fit
-};
-
-bool wave_shot(const ShotRun& R, WaveShot& W) {
+// Whether a shot runs through multi-step launches, and its splits.
+bool wave_shot(ShotRun& R) {
+  WaveShot& W = R.wave;
   const Prop& F = *R.F;
   const Prop& B = *R.B;
   if (R.fwd_unfused) return false;
@@ -2041,10 +2045,10 @@ bool wave_shot(const ShotRun& R, WaveShot& W) {
     W.f = W.alone;
     W.b = wave_plan(B, n, nb);
   }
-  return wave_wanted(W.alone) && wave_wanted(W.f) && wave_wanted(W.b);
+  W.on = wave_wanted(W.alone) && wave_wanted(W.f) && wave_wanted(W.b);
+  W.together = W.on && W.f.ctas() + W.b.ctas() <= sm_count() && !R.excitation && R.n_states > 1;
+  return W.on;
 }
-
-bool wave_together(const WaveShot& W) { return W.f.ctas() + W.b.ctas() <= sm_count(); }
 
 void wave_set_inject(WaveWork& w, ShotRun& R, const WavePlan& p) {
   if (!R.plan) return;
@@ -2064,7 +2068,7 @@ void wave_set_inject(WaveWork& w, ShotRun& R, const WavePlan& p) {
 void wave_add_replay(WaveRunner& run, ShotRun& R, const WavePlan& p, int b, int t, int n) {
   WaveWork& w = run.add(*R.F, p, n);
   w.t0 = t;
-  w.wavelet = R.wave.as<float>();
+  w.wavelet = R.wave_dev.as<float>();
   if (t == R.s_of(b)) {
     w.load = R.ck.as<float>() + (size_t)b * R.F->state_floats;
     R.F->step_index = R.ck_step[b];
@@ -2122,91 +2126,100 @@ void wave_finish_lowpass(ShotRun& R, int b, int t, double lowpass, cudaStream_t 
   if (e.kind != EPI_NONE) launch_epilogue(*R.B, e);
 }
 
-void wave_forward(WaveRunner& run, ShotRun& R, const WavePlan& p) {
+// Advance a shot by up to `budget` steps of its schedule: the forward pass
+// with checkpoints written by the launches themselves, then, block by block,
+// the replay of block b − 1 beside the backward pass over block b (two works
+// of one launch, two replay buffers) or one after the other; the excitation
+// condition maps the forward field, then runs backward.  Phases as in
+// ShotRun (4: done).
+void wave_advance(WaveRunner& run, ShotRun& R, int budget, cudaStream_t st) {
+  WaveShot& W = R.wave;
   Prop& F = *R.F;
-  for (int t = 0; t < R.nt; t += kWaveMaxSteps) {
-    const int m = std::min(kWaveMaxSteps, R.nt - t);
+  double lp = 0.0;
+  while (R.phase != 4 && budget > 0) {
+    const int most = std::min(budget, kWaveMaxSteps);
     run.begin();
-    WaveWork& w = run.add(F, p, m);
-    w.t0 = t;
-    w.wavelet = R.wave.as<float>();
-    w.ck = R.ck.as<float>();
-    w.ck_every = R.iv;
-    w.ck_floats = (int64_t)F.state_floats;
-    for (int b = (t + R.iv - 1) / R.iv; b < R.n_states && R.s_of(b) < t + m; ++b)
-      R.ck_step[b] = F.step_index + (R.s_of(b) - t) + 1;
-    F.step_index += m;
-    run.bytes = m * step_bytes(F);
-    run.launch();
+    if (R.phase == 0) {
+      const int t = R.t_f, m = std::min(most, R.nt - t);
+      WaveWork& w = run.add(F, W.whole, m);
+      w.t0 = t;
+      w.wavelet = R.wave_dev.as<float>();
+      w.ck = R.ck.as<float>();
+      w.ck_every = R.iv;
+      w.ck_floats = (int64_t)F.state_floats;
+      for (int b = (t + R.iv - 1) / R.iv; b < R.n_states && R.s_of(b) < t + m; ++b)
+        R.ck_step[b] = F.step_index + (R.s_of(b) - t) + 1;
+      F.step_index += m;
+      run.bytes = m * step_bytes(F);
+      run.launch();
+      budget -= m;
+      R.t_f += m;
+      if (R.t_f == R.nt) {
+        R.phase = R.excitation ? 2 : 1;
+        W.rb = W.bb = R.excitation ? 0 : R.n_states - 1;
+        W.rt = R.s_of(W.rb);
+        W.bt = R.e_of(W.bb) - 1;
+      }
+    } else if (R.phase == 2) {
+      const int n = std::min(most, R.e_of(W.rb) - W.rt);
+      wave_add_replay(run, R, W.alone, W.rb, W.rt, n);
+      run.launch();
+      budget -= n;
+      W.rt += n;
+      if (W.rt == R.e_of(W.rb) && ++W.rb == R.n_states) {
+        R.phase = 3;
+        W.bt = R.cfg.nt_spec - 1;
+      }
+    } else if (R.phase == 3) {
+      const int n = wave_add_backward(run, R, W.b, 0, W.bt, std::min(most, W.bt + 1), lp);
+      run.launch();
+      budget -= n;
+      W.bt -= n;
+      if (lp > 0.0) wave_finish_lowpass(R, 0, W.bt + 1, lp, st);
+      if (W.bt < 0) R.phase = 4;
+    } else {
+      // the backward pass over block b runs once block b is replayed; the
+      // replay stays at most one block ahead
+      const bool do_b = W.rb < W.bb;
+      const bool do_r = W.rb >= 0 && W.rb + (W.together ? 1 : 0) >= W.bb;
+      int nb = 0, nr = 0;
+      const int b_now = W.bb, t_now = W.bt;
+      lp = 0.0;
+      if (do_b) nb = wave_add_backward(run, R, W.b, W.bb, W.bt, std::min(most, W.bt - R.s_of(W.bb) + 1), lp);
+      if (do_r) {   // beside a backward segment, as many steps as it has
+        nr = std::min(R.e_of(W.rb) - W.rt, do_b ? nb : most);
+        wave_add_replay(run, R, do_b ? W.f : W.alone, W.rb, W.rt, nr);
+        W.rt += nr;
+        if (W.rt == R.e_of(W.rb)) {
+          --W.rb;
+          if (W.rb >= 0) W.rt = R.s_of(W.rb);
+        }
+      }
+      run.launch();
+      budget -= std::max(nb, nr);
+      if (do_b) {
+        W.bt -= nb;
+        if (lp > 0.0) wave_finish_lowpass(R, b_now, t_now - nb + 1, lp, st);
+        if (W.bt < R.s_of(W.bb)) {
+          --W.bb;
+          if (W.bb >= 0) W.bt = R.e_of(W.bb) - 1;
+          else R.phase = 4;
+        }
+      }
+    }
   }
 }
 
-bool migrate_wave(ShotRun& R, cudaStream_t st) {
-  WaveShot W;
-  if (!wave_shot(R, W)) return false;
-  WaveRunner run(st);
-  wave_forward(run, R, W.whole);
-  bool together = wave_together(W) && !R.excitation && R.n_states > 1;
-  if (together && !R.rbuf[1].p) {
-    try {
-      R.rbuf[1] = DevBuf(R.rbuf[0].bytes, st);
-    } catch (const Error&) {   // no room for a second replay buffer: one after the other
-      cudaGetLastError();
-      together = false;
-    }
+// A second replay buffer for a shot that runs side by side, if there is room;
+// else one after the other.
+void wave_second_buffer(ShotRun& R, cudaStream_t st) {
+  if (!R.wave.together || R.rbuf[1].p) return;
+  try {
+    R.rbuf[1] = DevBuf(R.rbuf[0].bytes, st);
+  } catch (const Error&) {
+    cudaGetLastError();
+    R.wave.together = false;
   }
-  double lp = 0.0;
-  if (R.excitation) {
-    for (int b = 0; b < R.n_states; ++b)
-      for (int t = R.s_of(b); t < R.e_of(b); t += kWaveMaxSteps) {
-        run.begin();
-        wave_add_replay(run, R, W.alone, b, t, std::min(kWaveMaxSteps, R.e_of(b) - t));
-        run.launch();
-      }
-    for (int t = R.cfg.nt_spec - 1; t >= 0;) {
-      run.begin();
-      const int n = wave_add_backward(run, R, W.b, 0, t, std::min(kWaveMaxSteps, t + 1), lp);
-      run.launch();
-      t -= n;
-      if (lp > 0.0) wave_finish_lowpass(R, 0, t + 1, lp, st);
-    }
-    return true;
-  }
-  // replay position and backward position; the backward pass over block b
-  // runs once block b is replayed, the replay stays at most one block ahead
-  int rb = R.n_states - 1, rt = R.s_of(rb), bb = rb, bt = R.e_of(rb) - 1;
-  while (bb >= 0) {
-    const bool can_b = rb < bb;
-    const bool can_r = rb >= 0 && rb + (together ? 1 : 0) >= bb;
-    run.begin();
-    const bool do_b = can_b;
-    const bool do_r = can_r;
-    int nb = 0;
-    const int b_now = bb, t_now = bt;
-    lp = 0.0;
-    if (do_b) nb = wave_add_backward(run, R, W.b, bb, bt, std::min(kWaveMaxSteps, bt - R.s_of(bb) + 1), lp);
-    if (do_r) {
-      // beside a backward segment, as many steps as it has
-      const int left = R.e_of(rb) - rt;
-      const int nr = do_b ? std::min(left, std::max(nb, 1)) : std::min(left, kWaveMaxSteps);
-      wave_add_replay(run, R, do_b ? W.f : W.alone, rb, rt, nr);
-      rt += nr;
-      if (rt == R.e_of(rb)) {
-        --rb;
-        if (rb >= 0) rt = R.s_of(rb);
-      }
-    }
-    run.launch();
-    if (do_b) {
-      bt -= nb;
-      if (lp > 0.0) wave_finish_lowpass(R, b_now, t_now - nb + 1, lp, st);
-      if (bt < R.s_of(bb)) {
-        --bb;
-        if (bb >= 0) bt = R.e_of(bb) - 1;
-      }
-    }
-  }
-  return true;
 }
 
 // Plain driver: one shot, steps one after the other (imaging.py:255-331).
@@ -2215,13 +2228,16 @@ void migrate(Prop& F, Prop& B, const ertm_migrate_config& cfg, const float* wave
   cudaStream_t st = F.st;
   ShotRun R;
   prepare_run(R, F, B, cfg, wavelet, record, num_out, illum_out, rillum_out, st, 1);
-  if (migrate_wave(R, st)) {
+  if (wave_shot(R)) {
+    wave_second_buffer(R, st);
+    WaveRunner run(st);
+    wave_advance(run, R, INT_MAX, st);
     CK(cudaGetLastError());
     finish_run(R, st);
     require_finite(R, st, "migrate");
     return;
   }
-  const float* dw = R.wave.as<float>();
+  const float* dw = R.wave_dev.as<float>();
   auto fwd_step = [&](int t, const Epilogue& e) {
     if (R.fwd_unfused) {
       step_once(F, 0.0, dw, t);
@@ -2541,7 +2557,7 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
     ShotRun& R = *Rp;
     switch (R.phase) {
       case 0: {  // forward with checkpoints
-        TickItem it{&R, true, make_work(*R.F, 0.0, R.wave.as<float>(), R.t_f, nullptr), false, {}};
+        TickItem it{&R, true, make_work(*R.F, 0.0, R.wave_dev.as<float>(), R.t_f, nullptr), false, {}};
         it.w.prop = R.fi;
         items.push_back(it);
         break;
@@ -2552,7 +2568,7 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
         if (do_rp) {
           if (R.rp_t == R.s_of(R.rp_block)) restores.push_back({&R, R.rp_block});
           Epilogue e = replay_epilogue(R, R.rp_block, R.rp_t);
-          TickItem it{&R, true, make_work(*R.F, 0.0, R.wave.as<float>(), R.rp_t, R.fwd_unfused ? nullptr : &e),
+          TickItem it{&R, true, make_work(*R.F, 0.0, R.wave_dev.as<float>(), R.rp_t, R.fwd_unfused ? nullptr : &e),
                       R.fwd_unfused, e};
           it.w.prop = R.fi;
           items.push_back(it);
@@ -2570,7 +2586,7 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
       case 2: {  // excitation map: replay every block forward
         if (R.rp_t == R.s_of(R.rp_block)) restores.push_back({&R, R.rp_block});
         Epilogue e = replay_epilogue(R, R.rp_block, R.rp_t);
-        TickItem it{&R, true, make_work(*R.F, 0.0, R.wave.as<float>(), R.rp_t, R.fwd_unfused ? nullptr : &e),
+        TickItem it{&R, true, make_work(*R.F, 0.0, R.wave_dev.as<float>(), R.rp_t, R.fwd_unfused ? nullptr : &e),
                     R.fwd_unfused, e};
         it.w.prop = R.fi;
         items.push_back(it);
@@ -2628,7 +2644,7 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
   for (TickItem& it : items) {
     ShotRun& R = *it.run;
     Prop& P = it.fwd ? *R.F : *R.B;
-    after_step(P, 0.0, it.fwd ? R.wave.as<float>() : nullptr, it.w.t, &lowpasses, it.unfused);
+    after_step(P, 0.0, it.fwd ? R.wave_dev.as<float>() : nullptr, it.w.t, &lowpasses, it.unfused);
   }
   if (!lowpasses.empty()) lowpass_props(lowpasses, st);
   // stand-alone epilogues: one launch per stencil order (k_epilogue_batch)
@@ -2703,9 +2719,27 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
   return true;
 }
 
+// Largest padded grid (cells) whose shots of a batch or session run through
+// multi-step launches, one after another, instead of in shared ticks.  A tick
+// costs much the same for any small grid, a multi-step launch follows the
+// cells: nine shots of three engines on 371–400 × 265–330 grids through the
+// serving loop 146 ms in ticks, 138 ms so; eight elastic 401×601 shots (0.25 M
+// cells) 101 ms in ticks, 119 ms so.
+constexpr int64_t kWaveBatchCells = 200000;
+
+bool wave_in_batch(ShotRun& R) {
+  const int mode = t_wave;
+  if (mode == 0 && (int64_t)R.F->h.nzp * R.F->h.nxp > kWaveBatchCells) return false;
+  return wave_shot(R);
+}
+
 void migrate_batch(std::vector<ShotRun>& runs, cudaStream_t st) {
   std::vector<ShotRun*> ptrs;
-  for (ShotRun& R : runs) ptrs.push_back(&R);
+  WaveRunner run(st);
+  for (ShotRun& R : runs) {
+    if (wave_in_batch(R)) wave_advance(run, R, INT_MAX, st);
+    else ptrs.push_back(&R);
+  }
   std::vector<DevProp> table;
   DevBuf dtable;
   upload_table(ptrs, table, dtable, st);
@@ -2715,6 +2749,8 @@ void migrate_batch(std::vector<ShotRun>& runs, cudaStream_t st) {
   std::string bad;
   for (size_t k = 0; k < runs.size(); ++k) {
     const uint32_t f = read_status(*runs[k].F, st), b = read_status(*runs[k].B, st);
+    if ((f | b) & STATUS_STALLED)
+      throw Error(ERTM_ERR_STATE, "migrate_batch: a wait between the CTAs of a launch ran out");
     if ((f | b) & STATUS_NONFINITE) bad += (bad.empty() ? "" : ", ") + std::to_string(k);
   }
   if (!bad.empty())
@@ -2735,6 +2771,7 @@ struct Session {
   DevBuf dtable, status;
   bool dirty = true;
   int64_t ticks = 0;
+  std::unique_ptr<WaveRunner> wave;   // exchange buffers of the shots in multi-step launches
 };
 
 // --------------------------------------------------------------------------
@@ -2986,7 +3023,7 @@ int32_t ertm_set_lane_assign(int32_t mode) {
 int32_t ertm_set_wave(int32_t mode) {
   return guarded([&] {
     REQUIRE(mode >= 0 && mode <= 2, "multi-step launches: 0 (automatic), 1 (never) or 2 (wherever they fit)");
-    g_wave.store(mode);
+    t_wave = mode;
   });
 }
 
@@ -3421,6 +3458,7 @@ int32_t ertm_session_add(void* session, const ertm_batch_shot* shot, int64_t tag
     auto R = std::make_unique<ShotRun>();
     prepare_run(*R, *static_cast<Prop*>(B.fwd), *static_cast<Prop*>(B.back), B.cfg, B.wavelet, B.record, B.num,
                 B.illum, B.rillum, S.st, 2);
+    wave_in_batch(*R);
     S.runs.push_back(std::move(R));
     S.tags.push_back(tag);
     S.dirty = true;
@@ -3432,10 +3470,14 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
     REQUIRE(session && n_done && max_ticks >= 0 && cap >= 0 && (done_tags || cap == 0), "bad arguments");
     Session& S = *static_cast<Session*>(session);
     *n_done = 0;
-    std::vector<ShotRun*> ptrs;
-    for (auto& R : S.runs) ptrs.push_back(R.get());
+    // shots in ticks, and shots in multi-step launches (as many steps each)
+    std::vector<ShotRun*> all, ptrs;
+    for (auto& R : S.runs) {
+      all.push_back(R.get());
+      if (!R->wave.on) ptrs.push_back(R.get());
+    }
     if (S.dirty) {
-      upload_table(ptrs, S.table, S.dtable, S.st);
+      upload_table(all, S.table, S.dtable, S.st);
       S.dirty = false;
     }
     auto any_done = [&] {
@@ -3443,6 +3485,10 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
         if (R->phase == 4) return true;
       return false;
     };
+    if (!S.wave) S.wave = std::make_unique<WaveRunner>(S.st);
+    for (ShotRun* R : all)
+      if (R->wave.on) wave_advance(*S.wave, *R, max_ticks, S.st);
+    if (ptrs.empty()) S.ticks += max_ticks;
     for (int k = 0; k < max_ticks && !any_done(); ++k) {
       if (!batch_tick(ptrs, S.dtable.as<DevProp>(), S.st)) break;
       ++S.ticks;
@@ -3458,6 +3504,8 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
       CK(cudaStreamSynchronize(S.st));
       for (size_t i = 0; i < S.runs.size();) {
         const ShotRun& R = *S.runs[i];
+        if ((flags[R.fi] | flags[R.bi]) & STATUS_STALLED)
+          throw Error(ERTM_ERR_STATE, "session: a wait between the CTAs of a launch ran out");
         if (!((flags[R.fi] | flags[R.bi]) & STATUS_NONFINITE)) {
           ++i;
           continue;

@@ -159,8 +159,9 @@ int32_t ertm_set_march(int32_t enable);
  * do not depend on it. */
 int32_t ertm_set_march_stress(int32_t enable);
 
-/* Multi-step launches (wavefields kept in shared memory over many steps):
- * 0 where they are expected to be faster, 1 never, 2 wherever they fit.
+/* Multi-step launches (wavefields kept in shared memory over many steps) in
+ * the calling thread's calls: 0 where they are expected to be faster, 1 never,
+ * 2 wherever they fit.
  * Results are identical in every mode. */
 int32_t ertm_set_wave(int32_t mode);
 /* Online autotuning of batched ticks (default on): the first ticks of each
