@@ -17,7 +17,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "ertm_b200" / "libertm_b200.so"
 SOURCES = [CSRC / "ertm_b200.cu", CSRC / "wave.cu"]
-DEPS = sorted(CSRC.glob("*.cu*")) + [HERE.parent / "include" / "ertm_b200.h"]
+DEPS = sorted(CSRC.glob("*.cu*")) + sorted(CSRC.glob("*.h")) + [HERE.parent / "include" / "ertm_b200.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

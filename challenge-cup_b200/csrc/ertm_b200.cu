@@ -432,7 +432,7 @@ struct InjectPlanHost {
   int n_cells = 0;
   std::vector<int32_t> h_field, h_index, h_start, h_src;   // host copies
   std::vector<double> h_wa, h_wb;
-  std::map<std::pair<int, int>, WaveInjectHost> wave;      // by (px, pz)
+  std::map<WaveKey, WaveInjectHost> wave;                  // by wave_key
   InjectPlanDev dev() const {
     InjectPlanDev d{};
     d.n_cells = n_cells;
@@ -444,20 +444,6 @@ struct InjectPlanHost {
     d.wb = wb.as<double>();
     return d;
   }
-};
-
-// How a propagator is split over at most `ncta` CTAs.
-struct WavePlan {
-  int px = 0, pz = 0;
-  int cells = 1;      // neighbouring cells of a thread's block
-  int thmax = 0, n_src = 0, n_acc = 0;
-  std::vector<int16_t> cut;
-  bool res = false;
-  int pad = 8;        // halo-field row padding (wave_layout)
-  int smem = 0;       // bytes
-  int64_t half = 0;   // exchange units per CTA and phase
-  bool ok() const { return px > 0; }
-  int ctas() const { return px * pz; }
 };
 
 struct Prop {
@@ -1662,7 +1648,6 @@ void require_finite(const ShotRun& R, cudaStream_t st, const std::string& what) 
 // For the calling thread's calls: 0 where they are expected to be faster;
 // 1 never; 2 wherever they fit.
 thread_local int t_wave = 0;
-constexpr int kWaveSmemMax = 227 * 1024 - 2048;   // dynamic shared memory (the static part left out)
 constexpr int kWaveMaxSteps = 1024;               // steps per launch: keeps a launch to a few ms
 
 int sm_count() {
@@ -1676,121 +1661,13 @@ int sm_count() {
   return n;
 }
 
-// What a work does besides stepping, for its shared memory: epilogue fields
-// (P, S), stored source fields read, imaging sums that could be resident.
-struct WaveNeeds {
-  int n_epi = 0, n_src = 0, n_acc = 0;
-};
-
-// Largest shared-memory need of a split, in bytes.
-int wave_smem(const DevProp& h, const WavePlan& p, const WaveNeeds& n) {
-  int most = 0;
-  for (int c = 0; c < p.px * p.pz; ++c) {
-    const WaveTile t = wave_tile(p.cut.data(), p.pz, p.px, c);
-    int f, nsx, nsz;
-    wave_strip(4 * t.g0, std::min(4 * (t.g0 + t.gw), h.nxp), h.nxp, h.npx_l, h.npx_r, f, nsx);
-    wave_strip(t.i0, t.i0 + t.th, h.nzp, h.npz_t, h.npz_b, f, nsz);
-    const WaveLayout y = wave_layout(h.engine == ENGINE_ELASTIC, h.engine == ENGINE_VISCO, h.L, p.res, p.pad, t.th,
-                                     t.gw, nsx, nsz, n.n_epi, p.n_src, p.n_acc);
-    most = std::max(most, y.total * 4);
-  }
-  return most;
-}
-
 bool wave_supported(const DevProp& h) {
   return h.M == 4 && h.fast_x == 1 && h.fast_z == 1 && h.nzp >= 8 && h.nxp >= 8 && h.nzp < 32768 && h.nxp < 32768 &&
          (h.engine != ENGINE_VISCO || h.L <= kRelaxUnroll);
 }
 
-// Cuts of n positions into k parts of about equal weight, each at least
-// `least` long; position q weighs weight(q).
-template <class F>
-void wave_cuts(int n, int k, int least, F&& weight, int16_t* cut) {
-  double total = 0.0;
-  for (int q = 0; q < n; ++q) total += weight(q);
-  double sum = 0.0;
-  int at = 0, first = 0;
-  cut[0] = 0;
-  for (int c = 0; c < k; ++c) {
-    const int last = n - least * (k - 1 - c);   // leave the later parts their least
-    while (at < last && (at - first < least || c + 1 == k || sum + 0.5 * weight(at) < total * (c + 1) / k)) {
-      sum += weight(at);
-      ++at;
-    }
-    cut[c + 1] = (int16_t)at;
-    first = at;
-  }
-}
-
-// Split over at most `ncta` CTAs.  Measured over px = 5 … 24 and strip weights
-// 0 … 2 on five grids: CTAs about 2.2 times as wide as tall are within 2 % of
-// the best, and so is a weight of 1.6 for CPML strips (their cells take the
-// general form and memory updates) with two cells a thread; with one cell a
-// thread (small grids, one pass of 512) 0.4.  Elastic 401×601 (µs a step):
-// 6.9 so, 7.9 with equal cuts, 11.6 the worst; acoustic 301×201 3.4 with one
-// cell a thread, 4.6 with two.  Imaging sums that do not fit in shared memory
-// cost about two round trips to L2 a step, coefficients that do not fit more.
-WavePlan make_wave_plan(const DevProp& h, int ncta, const WaveNeeds& n) {
-  WavePlan best;
-  if (!wave_supported(h)) return best;
-  const int ng = (h.nxp + 3) / 4, nx = h.engine == ENGINE_ELASTIC ? 2 : 1;
-  ncta = std::min(ncta, WAVE_MAX_CUTS - 4);
-  const double ideal = std::sqrt((double)h.nxp * ncta / (2.2 * h.nzp));
-  // cells per thread and pass; a split of one pass (WAVE_NT blocks a CTA at
-  // most) is cut for that rather than by weight
-  const double avg = (double)h.nzp * 4 * ng / (0.93 * WAVE_NT * ncta);
-  const int cells = avg <= 1.0 ? 1 : 2;
-  const bool single = avg <= 2.0;
-  double cost = 0.0;
-  for (const double strip : {single ? 0.4 : 1.6, 0.8, 0.0})
-  for (int px = std::max(1, std::min(ng, (int)ideal) - 2); px <= std::min({ncta, ng, (int)ideal + 3}); ++px) {
-    const int pz = std::min(ncta / px, h.nzp / WAVE_HALO);
-    if (pz < 1) continue;
-    auto row_w = [&](int i) { return i < h.npz_t || i >= h.nzp - h.npz_b ? 1.0 + strip : 1.0; };
-    auto col_w = [&](int g) {
-      int s = 0;
-      for (int j = 4 * g; j < 4 * g + 4; ++j) s += j < h.npx_l || (j >= h.nxp - h.npx_r && j < h.nxp) ? 1 : 0;
-      return 4.0 + strip * s;
-    };
-    WavePlan p;
-    p.px = px;
-    p.pz = pz;
-    p.cells = cells;
-    p.cut.resize(pz + px + 2);
-    wave_cuts(h.nzp, pz, WAVE_HALO, row_w, p.cut.data());
-    wave_cuts(ng, px, 1, col_w, p.cut.data() + pz + 1);
-    int gw = 0, most = 0;
-    for (int c = 0; c < p.ctas(); ++c) {
-      const WaveTile t = wave_tile(p.cut.data(), pz, px, c);
-      p.thmax = std::max(p.thmax, t.th);
-      gw = std::max(gw, t.gw);
-      most = std::max(most, t.th * t.gw * 4);
-    }
-    p.half = (int64_t)2 * nx * p.thmax + (int64_t)2 * nx * 4 * gw;
-    // the most that fits: resident coefficients first, then resident sums,
-    // then conflict-free rows
-    bool fits = false;
-    for (int k = 0; k < 8 && !fits; ++k) {
-      p.n_acc = (k & 2) == 0 ? n.n_acc : 0;
-      p.n_src = p.n_acc ? n.n_src : 0;
-      p.pad = (k & 1) == 0 ? 32 : 8;
-      p.res = k < 4;
-      p.smem = wave_smem(h, p, n);
-      fits = p.smem <= kWaveSmemMax;
-    }
-    if (!fits) continue;
-    // relative cost of a step: SMs left idle, the shape, equal cuts (measured
-    // 14 % with two cells a thread), a second pass of a few cells, sums and
-    // coefficients that do not fit
-    const double c = (double)ncta / p.ctas() * (1.0 + 0.03 * std::fabs(px - ideal)) *
-                     (single ? 1.0 + 0.05 * std::fabs(strip - 0.4) : 1.0 + 0.09 * (1.6 - strip)) *
-                     (single && most > WAVE_NT * cells ? 1.3 : 1.0) * (p.n_acc < n.n_acc ? 1.25 : 1.0) * (p.res ? 1.0 : 2.0);
-    if (!best.ok() || c < cost) {
-      best = p;
-      cost = c;
-    }
-  }
-  return best;
+WaveGrid wave_grid(const DevProp& h) {
+  return {h.engine == ENGINE_ELASTIC, h.engine == ENGINE_VISCO, h.L, h.nzp, h.nxp, h.npx_l, h.npx_r, h.npz_t, h.npz_b};
 }
 
 // The propagator's split, kept with it (0.1–0.5 ms to make; a function of the
@@ -1798,7 +1675,8 @@ WavePlan make_wave_plan(const DevProp& h, int ncta, const WaveNeeds& n) {
 const WavePlan& wave_plan(const Prop& P, int ncta, const WaveNeeds& n) {
   const std::array<int, 4> key{ncta, n.n_epi, n.n_src, n.n_acc};
   auto it = P.waves.find(key);
-  if (it == P.waves.end()) it = P.waves.emplace(key, make_wave_plan(P.h, ncta, n)).first;
+  if (it == P.waves.end())
+    it = P.waves.emplace(key, wave_supported(P.h) ? make_wave_plan(wave_grid(P.h), ncta, n) : WavePlan{}).first;
   return it->second;
 }
 
@@ -1859,23 +1737,10 @@ struct WaveRunner {
     epoch += 2 * (uint32_t)most + 2;
     cudaEvent_t e0 = nullptr;
     const bool timed = g_prof.begin(st, e0);
-    CK(wave_launch(engine, cells, res, S, grid, smem, kWaveSmemMax, st));
+    CK(wave_launch(engine, cells, res, S, grid, smem, WAVE_SMEM_MAX, st));
     ++g_launches;
     if (timed) g_prof.end(st, e0, bytes);
   }
-};
-
-// CTA of each padded cell's row and column group.
-struct WaveOwner {
-  std::vector<int> tr, tc;
-  int px;
-  WaveOwner(const DevProp& h, const WavePlan& p) : tr(h.nzp), tc((h.nxp + 3) / 4), px(p.px) {
-    for (int c = 0; c < p.pz; ++c)
-      for (int i = p.cut[c]; i < p.cut[c + 1]; ++i) tr[i] = c;
-    for (int c = 0; c < p.px; ++c)
-      for (int g = p.cut[p.pz + 1 + c]; g < p.cut[p.pz + 2 + c]; ++g) tc[g] = c;
-  }
-  int of(int i, int j) const { return tr[i] * px + tc[j / 4]; }
 };
 
 DevBuf wave_upload(const void* data, size_t bytes, cudaStream_t st) {
@@ -1885,25 +1750,19 @@ DevBuf wave_upload(const void* data, size_t bytes, cudaStream_t st) {
 }
 
 const WaveInjectHost& wave_inject(const Prop& P, InjectPlanHost& plan, const WavePlan& p) {
-  auto it = plan.wave.find({p.px, p.pz});   // a grid's cuts depend on these alone
+  const WaveKey key = wave_key(p);
+  auto it = plan.wave.find(key);
   if (it != plan.wave.end()) return it->second;
-  const WaveOwner own(P.h, p);
-  const int n = plan.n_cells, nc = p.ctas();
-  std::vector<int> cta(n);
-  std::vector<int32_t> first(nc + 1, 0);
-  for (int k = 0; k < n; ++k) {
-    cta[k] = own.of(plan.h_index[k] / P.h.ld, plan.h_index[k] % P.h.ld);
-    ++first[cta[k] + 1];
-  }
-  for (int c = 0; c < nc; ++c) first[c + 1] += first[c];
-  std::vector<int32_t> pos(first.begin(), first.end() - 1), order(n);
-  for (int k = 0; k < n; ++k) order[pos[cta[k]]++] = k;
+  const int n = plan.n_cells, ld = P.h.ld;
+  auto row_col = [&](int k) { return std::make_pair(plan.h_index[k] / ld, plan.h_index[k] % ld); };
+  const WaveGroups g = wave_groups(wave_grid(P.h), p, n, row_col);
   std::vector<int32_t> slot(n), ij(n), start{0}, src;
   std::vector<double> wa, wb;
   for (int q = 0; q < n; ++q) {
-    const int k = order[q];
+    const int k = g.order[q];
+    const auto [i, j] = row_col(k);
     slot[q] = plan.h_field[k];
-    ij[q] = (plan.h_index[k] / P.h.ld) << 16 | (plan.h_index[k] % P.h.ld);
+    ij[q] = i << 16 | j;
     for (int c = plan.h_start[k]; c < plan.h_start[k + 1]; ++c) {
       src.push_back(plan.h_src[c]);
       wa.push_back(plan.h_wa[c]);
@@ -1912,7 +1771,7 @@ const WaveInjectHost& wave_inject(const Prop& P, InjectPlanHost& plan, const Wav
     start.push_back((int32_t)src.size());
   }
   WaveInjectHost w;
-  w.cta = wave_upload(first.data(), first.size() * 4, P.st);
+  w.cta = wave_upload(g.first.data(), g.first.size() * 4, P.st);
   w.slot = wave_upload(slot.data(), slot.size() * 4, P.st);
   w.ij = wave_upload(ij.data(), ij.size() * 4, P.st);
   w.start = wave_upload(start.data(), start.size() * 4, P.st);
@@ -1920,7 +1779,7 @@ const WaveInjectHost& wave_inject(const Prop& P, InjectPlanHost& plan, const Wav
   w.wa = wave_upload(wa.data(), wa.size() * 8, P.st);
   w.wb = wave_upload(wb.data(), wb.size() * 8, P.st);
   CK(cudaStreamSynchronize(P.st));   // host vectors go out of scope
-  return plan.wave.emplace(std::make_pair(p.px, p.pz), std::move(w)).first->second;
+  return plan.wave.emplace(key, std::move(w)).first->second;
 }
 
 // Receiver sampling of a set of components: corner cells grouped by CTA.
@@ -1929,8 +1788,7 @@ struct WaveSampleHost {
 };
 
 WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& comps, const WavePlan& p) {
-  const WaveOwner own(P.h, p);
-  struct Entry { int cta, slot, ij, out; };
+  struct Entry { int slot, i, j, out; };
   std::vector<Entry> all;
   const int ld = P.h.ld;
   for (size_t c = 0; c < comps.size(); ++c) {
@@ -1938,26 +1796,21 @@ WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& co
     if (sp.kind == SAMPLE_ZERO) continue;
     for (int r = 0; r < sp.n; ++r) {
       if (!sp.h_valid[r]) continue;
-      for (int corner = 0; corner < 4; ++corner) {
-        const int i = sp.h_cell[r] / ld + (corner >> 1), j = sp.h_cell[r] % ld + (corner & 1);
-        all.push_back({own.of(i, j), sp.kind == SAMPLE_PRESSURE ? -1 : sp.slot, i << 16 | j,
-                       4 * ((int)c * sp.n + r) + corner});
-      }
+      for (int corner = 0; corner < 4; ++corner)
+        all.push_back({sp.kind == SAMPLE_PRESSURE ? -1 : sp.slot, sp.h_cell[r] / ld + (corner >> 1),
+                       sp.h_cell[r] % ld + (corner & 1), 4 * ((int)c * sp.n + r) + corner});
     }
   }
-  const int nc = p.ctas();
-  std::vector<int32_t> first(nc + 1, 0), slot(all.size()), ij(all.size()), out(all.size());
-  for (const Entry& e : all) ++first[e.cta + 1];
-  for (int c = 0; c < nc; ++c) first[c + 1] += first[c];
-  std::vector<int32_t> pos(first.begin(), first.end() - 1);
-  for (const Entry& e : all) {
-    const int q = pos[e.cta]++;
-    slot[q] = e.slot;
-    ij[q] = e.ij;
-    out[q] = e.out;
+  const WaveGroups g = wave_groups(wave_grid(P.h), p, (int)all.size(),
+                                   [&](int k) { return std::make_pair(all[k].i, all[k].j); });
+  std::vector<int32_t> slot, ij, out;
+  for (const int32_t k : g.order) {
+    slot.push_back(all[k].slot);
+    ij.push_back(all[k].i << 16 | all[k].j);
+    out.push_back(all[k].out);
   }
   WaveSampleHost w;
-  w.cta = wave_upload(first.data(), first.size() * 4, P.st);
+  w.cta = wave_upload(g.first.data(), g.first.size() * 4, P.st);
   w.slot = wave_upload(slot.data(), slot.size() * 4, P.st);
   w.ij = wave_upload(ij.data(), ij.size() * 4, P.st);
   w.out = wave_upload(out.data(), out.size() * 4, P.st);

@@ -50,102 +50,12 @@
 #include <type_traits>
 
 #include "step_kernels.cuh"
+#include "wave_plan.h"
 
 namespace ertm {
 
-constexpr int WAVE_NT = 512;
 constexpr int WAVE_MAX_WORKS = 16;
 constexpr int WAVE_SPIN_LIMIT = 1 << 20;   // polls of one packet (about a second)
-constexpr int WAVE_HALO = 4;
-
-// Rows [i0, i0 + th) and column groups [g0, g0 + gw) of CTA c of a pz × px
-// split with row cuts cut[0 … pz] and column-group cuts cut[pz + 1 …].
-struct WaveTile {
-  int i0, th, g0, gw, tr, tc;
-};
-__host__ __device__ inline WaveTile wave_tile(const int16_t* cut, int pz, int px, int c) {
-  WaveTile t;
-  t.tr = c / px;
-  t.tc = c - t.tr * px;
-  t.i0 = cut[t.tr];
-  t.th = cut[t.tr + 1] - t.i0;
-  t.g0 = cut[pz + 1 + t.tc];
-  t.gw = cut[pz + 2 + t.tc] - t.g0;
-  return t;
-}
-constexpr int WAVE_MAX_CUTS = 160;   // pz + px + 2 of a split over up to 156 CTAs
-
-// Strip columns / rows of [lo, hi) in ψ-array coordinates: first index and count.
-__host__ __device__ inline void wave_strip(int lo, int hi, int n, int a, int b, int& first, int& count) {
-  // strip index of position q: q for q < a, a + q − (n − b) for q ≥ n − b
-  const int l0 = lo < a ? lo : a, l1 = hi < a ? hi : a;
-  const int r0 = lo > n - b ? lo : n - b, r1 = hi < n ? hi : n;
-  const int nl = l1 > l0 ? l1 - l0 : 0, nr = r1 > r0 ? r1 - r0 : 0;
-  first = nl > 0 ? l0 : a + (r0 - (n - b));
-  count = nl + nr;
-  if (count == 0) first = 0;
-}
-
-// Shared-memory layout of one CTA, in floats from the start of dynamic shared
-// memory (every array a multiple of 16 bytes).
-struct WaveLayout {
-  int W, H, cw;          // halo-field pitch and rows, cell-array pitch
-  int field, field_n;    // halo fields, floats per field
-  int cell, cell_n;      // per-cell arrays, floats per array
-  int qidx;              // viscoacoustic Q index bytes
-  int epi;               // P (and S) of the last step for the epilogue
-  int src;               // stored source fields of the last step
-  int acc;               // imaging sums, two floats a cell each
-  int psix, psix_n;      // x-strip memories (pitch nsx), floats per term
-  int psiz, psiz_n;      // z-strip memories (pitch cw), floats per term
-  int col, row;          // per column / row: profile a, b, strip index and flags
-  int units, units_n;    // exchange tables (int4 per unit, two phases)
-  int total;
-};
-
-__host__ __device__ inline int wave_r4(int n) { return (n + 3) / 4 * 4; }
-
-// pad: floats between the rows of a halo field beyond its own cells.  8 holds
-// the halo; with 32 the rows' first cells continue the bank sequence of the
-// cells before them, so a warp that spans rows has no bank conflicts.
-__host__ __device__ inline WaveLayout wave_layout(bool elastic, bool visco, int L, bool res, int pad, int th, int gw,
-                                                  int nsx, int nsz, int n_epi, int n_src, int n_acc) {
-  WaveLayout y;
-  const int nf = elastic ? 5 : 3, nx = elastic ? 2 : 1, n_psi = elastic ? 4 : 2;
-  y.cw = 4 * gw;
-  y.W = y.cw + pad;
-  y.H = th + 2 * WAVE_HALO;
-  int o = 0;
-  y.field = o;
-  y.field_n = y.W * y.H;
-  o += nf * y.field_n;
-  y.cell = o;
-  y.cell_n = th * y.cw;
-  o += res ? (visco ? 4 + 2 * L : (elastic ? 5 : 3)) * y.cell_n : 0;
-  y.qidx = o;
-  o += res && visco ? wave_r4(th * gw) : 0;   // one byte per cell
-  y.epi = o;
-  o += n_epi * y.cell_n;
-  y.src = o;
-  o += n_src * y.cell_n;
-  y.acc = o;
-  o += 2 * n_acc * y.cell_n;
-  y.psix = o;
-  y.psix_n = res ? wave_r4(th * nsx) : 0;
-  o += n_psi * y.psix_n;
-  y.psiz = o;
-  y.psiz_n = res ? nsz * y.cw : 0;
-  o += n_psi * y.psiz_n;
-  y.col = o;
-  o += 4 * y.cw;
-  y.row = o;
-  o += 4 * th;
-  y.units_n = 2 * nx * th + 2 * nx * 4 * gw;
-  y.units = o;
-  o += 2 * 4 * y.units_n;
-  y.total = o;
-  return y;
-}
 
 // One exchange unit: four cells of one field on one side of a CTA.  It sends
 // own cells `src` and receives into halo cells `dst` (offsets from own cell
