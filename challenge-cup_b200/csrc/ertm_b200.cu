@@ -1444,6 +1444,7 @@ struct ShotRun {
   int phase = 0;
   int t_f = 0, rp_block = -1, rp_t = 0, bk_block = -1, bk_t = 0, replayed_below = 0;
   WaveShot wave;
+  bool routed = false;         // a session's shot: the route is chosen (see wave_in_batch)
   int s_of(int b) const { return b * iv; }
   int e_of(int b) const { return std::min((b + 1) * iv, nt); }
 };
@@ -2572,25 +2573,21 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
   return true;
 }
 
-// Largest padded grid (cells) whose shots of a batch or session run through
-// multi-step launches, one after another, instead of in shared ticks.  A tick
-// costs much the same for any small grid, a multi-step launch follows the
-// cells: nine shots of three engines on 371–400 × 265–330 grids through the
-// serving loop 146 ms in ticks, 138 ms so; eight elastic 401×601 shots (0.25 M
-// cells) 101 ms in ticks, 119 ms so.
-constexpr int64_t kWaveBatchCells = 200000;
-
-bool wave_in_batch(ShotRun& R) {
-  const int mode = t_wave;
-  if (mode == 0 && (int64_t)R.F->h.nzp * R.F->h.nxp > kWaveBatchCells) return false;
+// Whether a shot of a batch or session runs through multi-step launches, with
+// `together` shots of its engine in flight, itself included.
+bool wave_in_batch(ShotRun& R, int together) {
+  const DevProp& h = R.F->h;
+  if (t_wave == 0 && !wave_few(h.engine == ENGINE_VISCO, (int64_t)h.nzp * h.nxp, together)) return false;
   return wave_shot(R);
 }
 
 void migrate_batch(std::vector<ShotRun>& runs, cudaStream_t st) {
   std::vector<ShotRun*> ptrs;
   WaveRunner run(st);
+  int count[3] = {};   // shots per engine
+  for (ShotRun& R : runs) ++count[R.F->h.engine];
   for (ShotRun& R : runs) {
-    if (wave_in_batch(R)) wave_advance(run, R, INT_MAX, st);
+    if (wave_in_batch(R, count[R.F->h.engine])) wave_advance(run, R, INT_MAX, st);
     else ptrs.push_back(&R);
   }
   std::vector<DevProp> table;
@@ -3311,7 +3308,6 @@ int32_t ertm_session_add(void* session, const ertm_batch_shot* shot, int64_t tag
     auto R = std::make_unique<ShotRun>();
     prepare_run(*R, *static_cast<Prop*>(B.fwd), *static_cast<Prop*>(B.back), B.cfg, B.wavelet, B.record, B.num,
                 B.illum, B.rillum, S.st, 2);
-    wave_in_batch(*R);
     S.runs.push_back(std::move(R));
     S.tags.push_back(tag);
     S.dirty = true;
@@ -3323,9 +3319,16 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
     REQUIRE(session && n_done && max_ticks >= 0 && cap >= 0 && (done_tags || cap == 0), "bad arguments");
     Session& S = *static_cast<Session*>(session);
     *n_done = 0;
-    // shots in ticks, and shots in multi-step launches (as many steps each)
+    // shots in ticks, and shots in multi-step launches (as many steps each); a
+    // shot keeps the route it gets when it first advances
+    int count[3] = {};   // shots in flight per engine
+    for (auto& R : S.runs) ++count[R->F->h.engine];
     std::vector<ShotRun*> all, ptrs;
     for (auto& R : S.runs) {
+      if (!R->routed) {
+        wave_in_batch(*R, count[R->F->h.engine]);
+        R->routed = true;
+      }
       all.push_back(R.get());
       if (!R->wave.on) ptrs.push_back(R.get());
     }

@@ -243,6 +243,26 @@ inline WavePlan make_wave_plan(const WaveGrid& h, int ncta, const WaveNeeds& n) 
   return best;
 }
 
+// Whether a shot of a batch or session runs through multi-step launches, one
+// shot after another, rather than in ticks that all shots share: `cells` of its
+// padded grid, `together` shots of its engine in flight.  A tick's launches
+// cost much the same for one small shot as for several, a multi-step launch
+// follows the shots.  Ticks over multi-step launches, times of 200 steps of
+// batches on 256×256 to 440×440 grids:
+//
+//   shots           1          2          3          4          8         16         45
+//   acoustic        1.7–2.0    1.2–1.6    1.07–1.12  0.96–1.13  0.86–0.93 0.76–0.89  0.78–0.91
+//   elastic         1.5–1.9    1.2–1.4    0.97–1.04  0.88–0.99  0.76–0.82 0.70–0.74  0.73–0.75
+//   viscoacoustic   1.4–1.8    1.02–1.2   0.82–0.95  0.80–0.98  0.67–0.72 0.63–0.74  0.64–0.75
+//
+// (a viscoacoustic tick's low-passes share their transforms' launches).  Above
+// 200,000 cells two shots of an engine come out between 0.94 and 1.5; those
+// keep the ticks.  45 shots in flight in the serving loop: 32.5 shots/s in
+// ticks, 28.6 in multi-step launches.
+inline bool wave_few(bool visco, int64_t cells, int together) {
+  return cells <= 200000 && together <= (visco ? 2 : 3);
+}
+
 // CTA of each padded cell's row and column group.
 struct WaveOwner {
   std::vector<int> tr, tc;

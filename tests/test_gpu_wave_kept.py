@@ -79,3 +79,19 @@ def test_kept_batch_with_other_modes(order):
         for x, y in zip(got, want, strict=True):
             for a, b in zip(_images(x), _images(y), strict=True):
                 assert np.array_equal(a, b), modes
+
+
+def test_session_of_both_routes_gives_one_shot_images():
+    """Few shots of one engine beside many of another, more of them joining: ticks and multi-step launches in one
+    session."""
+    from ertm_b200.serving import RTMServer, ServeJob
+    jobs = []
+    for engine, boundary, n in (("elastic", "free", 2), ("viscoacoustic", "cpml", 5), ("acoustic", "free", 4)):
+        model, shot = _shot((96, 140), engine, boundary)
+        jobs += [(_imager(engine, boundary, shot.dt), model, shot)] * n
+    want = {id(model): _images(imager.migrate_modes(shot, model)) for imager, model, shot in jobs}
+    with RTMServer(max_shots=7, ticks_per_poll=16) as server:
+        futures = [server.submit(ServeJob(shots=[shot], model=model, imager=imager)) for imager, model, shot in jobs]
+        for f, (_, model, _) in zip(futures, jobs):
+            for r, b in zip(f.result(timeout=120).images, want[id(model)], strict=True):
+                assert np.array_equal(r.image, b)

@@ -7,7 +7,7 @@ import itertools
 import numpy as np
 import pytest
 
-from wave_split import split
+from wave_split import few_shots, split
 
 # what a work keeps in shared memory beside the fields: (P/S fields, stored source fields, imaging sums)
 _NEEDS = {"acoustic": [(0, 0, 0), (0, 1, 1), (0, 1, 2), (0, 1, 3)],
@@ -46,3 +46,11 @@ def test_grouped_points_lie_in_their_tile(engine):
         tr, tc = cta // p.px, cta % p.px
         assert (p.rows[tr] <= i).all() and (i < p.rows[tr + 1]).all()
         assert (p.groups[tc] <= g).all() and (g < p.groups[tc + 1]).all()
+
+
+@pytest.mark.parametrize("engine", sorted(_NEEDS))
+def test_many_shots_share_ticks(engine):
+    """A batch or a loaded server advances its shots in common ticks; one or two small shots run alone."""
+    for nz, nx in ((256, 256), (330, 400)):
+        assert all(few_shots(engine, nz, nx, n) for n in (1, 2))
+        assert not any(few_shots(engine, nz, nx, n) for n in (4, 8, 45))

@@ -33,6 +33,7 @@ extern "C" int wave_split(const int* g, int ncta, const int* n, int* out, int16_
   std::copy(q.order.begin(), q.order.end(), order);
   return (int)k.size();
 }
+extern "C" int wave_few_shots(int visco, int64_t cells, int together) { return wave_few(visco != 0, cells, together); }
 """
 
 
@@ -83,3 +84,8 @@ def split(engine: str, nz: int, nx: int, *, npml: int = 20, boundary: str = "cpm
     cuts = np.array(cut[: px + pz + 2])
     return Split(px, pz, out[2], bool(out[3]), out[4], out[5], cuts[: pz + 1], cuts[pz + 1:], tuple(key[:k]),
                  first[: px * pz + 1], order[: rows.size])
+
+
+def few_shots(engine: str, nz: int, nx: int, together: int) -> bool:
+    """Whether shots of a batch or session take multi-step launches."""
+    return bool(_shim().wave_few_shots(int(engine == "viscoacoustic"), C.c_int64((nz + 10) * (nx + 10)), together))
