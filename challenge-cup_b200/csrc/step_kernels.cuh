@@ -384,6 +384,12 @@ __device__ __forceinline__ void acc_term(double* base, int kahan, size_t c, size
   }
 }
 
+// GATHER: the Kahan sums of an image in flight together (six acoustic and
+// elastic shots of four grids 159 → 150 ms).  Off where the registers that
+// takes would cost float64 runs: the 32-row elastic frame kernel (124
+// registers; 160 with it, or spills under a cap: eight 401×601 shots with
+// float64 sums 96 → 98 ms) and the marching kernels.
+template <bool GATHER = true>
 __device__ __forceinline__ void run_epilogue(const Epilogue& E, size_t c, size_t npix, float pv, float sv) {
   switch (E.kind) {
     case EPI_STORE:
@@ -417,37 +423,37 @@ __device__ __forceinline__ void run_epilogue(const Epilogue& E, size_t c, size_t
         }
         break;
       }
-      // Kahan sums: likewise every sum and compensation first, then acc_term's
-      // update of each
-      float a[3][MAX_EPI_IMAGES], q[3][MAX_EPI_IMAGES];
-      auto sum_of = [&](int kind, int k) -> float* {   // S², R², S·R
-        return reinterpret_cast<float*>(kind == 0 ? (E.illum ? E.ill[k] : nullptr)
-                                                  : (kind == 1 ? (E.rillum ? E.ril[k] : nullptr)
-                                                               : (E.cross ? E.num[k] : nullptr)));
-      };
-#pragma unroll
-      for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
-        if (k >= E.n_images) break;
-#pragma unroll
-        for (int kind = 0; kind < 3; ++kind)
-          if (const float* p = sum_of(kind, k)) {
-            a[kind][k] = p[c];
-            q[kind][k] = p[npix + c];
-          }
-      }
+      // Kahan sums: with GATHER the sums and compensations of an image are
+      // loaded before any is stored, then acc_term's update of each
 #pragma unroll
       for (int k = 0; k < MAX_EPI_IMAGES; ++k) {
         if (k >= E.n_images) break;
         const float s = E.src_slot[k] ? s1 : s0;
         const float r = E.rcv_wave[k] ? sv : pv;
+        if constexpr (!GATHER) {
+          if (E.illum && E.ill[k]) acc_term(E.ill[k], 1, c, npix, fmul(s, s));
+          if (E.rillum && E.ril[k]) acc_term(E.ril[k], 1, c, npix, fmul(r, r));
+          if (E.cross) acc_term(E.num[k], 1, c, npix, fmul(s, r));
+        } else {
+          float* const p[3] = {reinterpret_cast<float*>(E.illum ? E.ill[k] : nullptr),
+                               reinterpret_cast<float*>(E.rillum ? E.ril[k] : nullptr),
+                               reinterpret_cast<float*>(E.cross ? E.num[k] : nullptr)};
+          float a[3], q[3];
 #pragma unroll
-        for (int kind = 0; kind < 3; ++kind)
-          if (float* p = sum_of(kind, k)) {
-            const float term = kind == 0 ? fmul(s, s) : (kind == 1 ? fmul(r, r) : fmul(s, r));
-            const float y = fsub(term, q[kind][k]), t = fadd(a[kind][k], y);
-            p[npix + c] = fsub(fsub(t, a[kind][k]), y);
-            p[c] = t;
-          }
+          for (int n = 0; n < 3; ++n)
+            if (p[n]) {
+              a[n] = p[n][c];
+              q[n] = p[n][npix + c];
+            }
+#pragma unroll
+          for (int n = 0; n < 3; ++n)
+            if (p[n]) {
+              const float term = n == 0 ? fmul(s, s) : (n == 1 ? fmul(r, r) : fmul(s, r));
+              const float y = fsub(term, q[n]), t = fadd(a[n], y);
+              p[n][npix + c] = fsub(fsub(t, a[n]), y);
+              p[n][c] = t;
+            }
+        }
       }
       break;
     }
@@ -572,7 +578,7 @@ __device__ __forceinline__ void prefetch_image_tile(const Epilogue& E, const GEO
   }
 }
 
-template <int TZ, int NT, class GEO>
+template <int TZ, int NT, bool GATHER = true, class GEO>
 __device__ __forceinline__ void epilogue_tile(const Epilogue& E, const GEO& G, int i0, int j0, const float* e_p,
                                               const float* e_s, size_t npix) {
   if (E.kind == EPI_IMAGE && !E.kahan && (TZ * 32) % NT == 0) {
@@ -583,7 +589,7 @@ __device__ __forceinline__ void epilogue_tile(const Epilogue& E, const GEO& G, i
 #pragma unroll 1
   for (int idx = tid; idx < TZ * 32; idx += NT) {
     size_t pc;
-    if (G.physical(i0 + (idx >> 5), j0 + (idx & 31), pc)) run_epilogue(E, pc, npix, e_p[idx], e_s ? e_s[idx] : 0.f);
+    if (G.physical(i0 + (idx >> 5), j0 + (idx & 31), pc)) run_epilogue<GATHER>(E, pc, npix, e_p[idx], e_s ? e_s[idx] : 0.f);
   }
 }
 
@@ -1111,12 +1117,6 @@ __device__ __forceinline__ void block_max_to(float v, float* dst) {
 template <bool VISCO, int KIND, int R>
 constexpr int kStressMinBlocks = (VISCO && KIND == TILES_INTERIOR && R == 1) ? 9 : 1;
 
-// Resident blocks per SM the elastic stress kernels are compiled for (0: the
-// compiler's own choice): the 32-row frame kernel takes 160 registers uncapped
-// (3 blocks), 128 capped for 4.
-template <int KIND, int R>
-constexpr int kElasticMinBlocks = (KIND == TILES_FRAME && R == 2) ? 4 : 0;
-
 // Acoustic (VISCO=false): p += (dt·κ)·div.  Viscoacoustic (VISCO=true):
 // ε += dt·div; r_l ← r_l·a_l + b_l·Δε; p = K_R·ε + Σ r_l.
 template <int M, int BZ, int R, bool VISCO, int KIND, class WS, class TM>
@@ -1313,7 +1313,7 @@ k_pressure_stress(const DevProp* __restrict__ props, const WS ws, const __grid_c
 // then the epilogue with P/S from the stresses (stress separation) or from
 // the raw velocity divergence/curl (divcurl, propagation.py:953-976).
 template <int M, int BZ, int R, int KIND, class WS, class TM>
-__global__ void __launch_bounds__(XT* BZ, kElasticMinBlocks<KIND, R>)
+__global__ void __launch_bounds__(XT* BZ)
 k_elastic_stress(const DevProp* __restrict__ props, const WS ws, const __grid_constant__ TM tm) {
   constexpr int TZ = BZ * R;
   using T = TileShape<M, TZ>;
@@ -1540,7 +1540,7 @@ k_elastic_stress(const DevProp* __restrict__ props, const WS ws, const __grid_co
   }
   if (epi && valid) {
     __syncthreads();
-    epilogue_tile<TZ, XT * BZ>(E, G, L.i0, L.j0, e_p, e_s, npix);
+    epilogue_tile<TZ, XT * BZ, !(KIND == TILES_FRAME && R == 2)>(E, G, L.i0, L.j0, e_p, e_s, npix);
   }
 }
 
@@ -1842,7 +1842,7 @@ k_elastic_stress_march(const DevProp* __restrict__ props, const WS ws) {
     }
     if (epi && run) {
       __syncthreads();
-      epilogue_tile<MARCH_CH, NT>(E, G, a, j0, cell_b[b][0], cell_b[b][1], npix);
+      epilogue_tile<MARCH_CH, NT, false>(E, G, a, j0, cell_b[b][0], cell_b[b][1], npix);
     }
     __syncthreads();   // the next iteration refills this chunk's buffers
   }
