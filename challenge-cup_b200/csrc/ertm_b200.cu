@@ -1688,8 +1688,7 @@ struct WaveRunner {
   DevBuf xbuf, peaks;
   uint32_t epoch = 0;
   WaveSet S{};
-  int grid = 0, smem = 0, engine = 0, cells = 1;
-  bool res = true;            // the works of a launch share engine, cells and res
+  int grid = 0, smem = 0, engine = 0, cells = 1;   // shared by the works of a launch
   double bytes = 0.0;
   explicit WaveRunner(cudaStream_t s) : st(s) {}
   void begin() {
@@ -1702,7 +1701,6 @@ struct WaveRunner {
     WaveWork& w = S.w[S.n++];
     engine = P.h.engine;
     cells = p.cells;
-    res = p.res;
     w.prop = P.dp();
     w.cta0 = grid;
     w.px = p.px;
@@ -1738,7 +1736,7 @@ struct WaveRunner {
     epoch += 2 * (uint32_t)most + 2;
     cudaEvent_t e0 = nullptr;
     const bool timed = g_prof.begin(st, e0);
-    CK(wave_launch(engine, cells, res, S, grid, smem, WAVE_SMEM_MAX, st));
+    CK(wave_launch(engine, cells, S, grid, smem, WAVE_SMEM_MAX, st));
     ++g_launches;
     if (timed) g_prof.end(st, e0, bytes);
   }
@@ -1819,12 +1817,8 @@ WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& co
   return w;
 }
 
-// Grids the multi-step launches are used for: whatever fits with the
-// coefficients resident.
-bool wave_wanted(const WavePlan& p) {
-  const int mode = t_wave;
-  return p.ok() && mode != 1 && (mode == 2 || p.res);
-}
+// Grids the multi-step launches are used for: whatever fits.
+bool wave_wanted(const WavePlan& p) { return p.ok() && t_wave != 1; }
 
 // Forward modelling through multi-step launches; false when the propagator
 // does not qualify.
@@ -1894,7 +1888,7 @@ bool wave_shot(ShotRun& R) {
   W.alone = wave_plan(F, n, nf);
   W.f = wave_plan(F, n / 2, nf);
   W.b = wave_plan(B, n / 2, nb);
-  if (!W.f.ok() || !W.b.ok() || W.f.res != W.b.res || !W.f.res || W.f.cells != W.b.cells ||
+  if (!W.f.ok() || !W.b.ok() || W.f.cells != W.b.cells ||
       (W.b.n_acc < nb.n_acc && wave_plan(B, n, nb).n_acc == nb.n_acc)) {
     W.f = W.alone;
     W.b = wave_plan(B, n, nb);

@@ -732,9 +732,7 @@ __device__ __forceinline__ ColInfo col_info(const Geo& G, int j, const float* ax
 // mechanism costs two vector loads and one vector store.  Columns with
 // keep[c] set are left as they are.  Up to kRelaxUnroll mechanisms run
 // unrolled.
-// SHARED: b_l lies in shared memory (not readable through the read-only path).
 constexpr int kRelaxUnroll = 4;
-template <bool SHARED = false>
 __device__ __forceinline__ void relax4(float* r0, const float* b0, size_t fstride, const uint8_t* qidx,
                                        const float* relax_a, int nL, size_t g, const float (&inc)[4],
                                        const bool (&keep)[4], float (&tot)[4]) {
@@ -752,7 +750,7 @@ __device__ __forceinline__ void relax4(float* r0, const float* b0, size_t fstrid
     for (int l = 0; l < kRelaxUnroll; ++l) {
       if (l < nL) {
         r4[l] = ld4(r0 + l * fstride + g);
-        b4[l] = SHARED ? ld4(b0 + l * fstride + g) : ldg4(b0 + l * fstride + g);
+        b4[l] = ldg4(b0 + l * fstride + g);
       }
     }
 #pragma unroll
@@ -773,7 +771,7 @@ __device__ __forceinline__ void relax4(float* r0, const float* b0, size_t fstrid
   for (int l = 0; l < nL; ++l) {
     float* rl = r0 + l * fstride;
     const float4 r4 = ld4(rl + g);
-    const float4 b4 = SHARED ? ld4(b0 + l * fstride + g) : ldg4(b0 + l * fstride + g);
+    const float4 b4 = ldg4(b0 + l * fstride + g);
     float4 o4;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {

@@ -10,10 +10,10 @@
 // stencils read:
 //
 //  * a CTA owns a rectangle of rows × 4-column groups of the padded grid.  The
-//    fields a stencil reads live in shared memory with a four-cell halo; with
-//    RES, so do the per-cell coefficients (those that meet dt as a product
-//    already multiplied by it), the CPML memories and the viscoacoustic ε and
-//    r_l, and a step touches global memory only for edges, images, samples.
+//    fields a stencil reads live in shared memory with a four-cell halo, and so
+//    do the per-cell coefficients (those that meet dt as a product already
+//    multiplied by it), the CPML memories and the viscoacoustic ε and r_l: a
+//    step touches global memory only for edges, images and samples.
 //  * edges travel through L2 as units of four values, each value in one
 //    64-bit word with the exchange's number (epoch): a reader polls the words
 //    themselves, so an exchange needs no fence and no flag, and a word of an
@@ -54,7 +54,7 @@
 
 namespace ertm {
 
-constexpr int WAVE_MAX_WORKS = 16;
+constexpr int WAVE_MAX_WORKS = 2;     // a shot's replay beside its backward pass
 constexpr int WAVE_SPIN_LIMIT = 1 << 20;   // polls of one packet (about a second)
 
 // One exchange unit: four cells of one field on one side of a CTA.  It sends
@@ -462,9 +462,8 @@ constexpr int WAVE_SURFACE = 4;   // the free-surface row
 __device__ __forceinline__ int wave_strip_of(const float4& t) { return __float_as_int(t.z); }
 __device__ __forceinline__ int wave_flags_of(const float4& t) { return __float_as_int(t.w); }
 
-// ENG: Engine; C: neighbouring cells a thread updates together; RES: per-cell coefficients (and viscoacoustic ε, r_l) in
-// shared memory, else read from and written to global memory every step.
-template <int ENG, int C, bool RES>
+// ENG: Engine; C: neighbouring cells a thread updates together.
+template <int ENG, int C>
 __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ WaveSet S) {
   constexpr int M = 4;
   static_assert(C == 1 || C == 2, "one or two cells per thread");
@@ -504,7 +503,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   wave_strip(i0, i0 + th, G.nzp, G.npz_t, G.npz_b, sz0, nsz);
   const int ekind = w.epi.kind;
   const int n_epi = (!EL || ekind == EPI_NONE) ? 0 : (w.epi.need_s ? 2 : 1);   // P and S kept beside the fields
-  const WaveLayout Y = wave_layout(EL, VISCO, nL, RES, w.pad, th, gw, nsx, nsz, n_epi, w.n_src, w.n_acc);
+  const WaveLayout Y = wave_layout(EL, VISCO, nL, w.pad, th, gw, nsx, nsz, n_epi, w.n_src, w.n_acc);
   const int W = Y.W, cw = Y.cw;
   float* const own = sm + Y.field + WAVE_HALO * W + WAVE_HALO;   // own cell (0, 0) of field 0
   const int FN = Y.field_n;
@@ -517,27 +516,18 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   float* const accs = sm + Y.acc;
   const float4* const coltab = reinterpret_cast<const float4*>(sm + Y.col);
   const float4* const rowtab = reinterpret_cast<const float4*>(sm + Y.row);
-  // ψ of x term t at (row r, strip column s): psx(t)[r·pxw + s]; of z term t
-  // at (strip row s, tile column c): psz(t)[s·pzw + c]
-  const int pxw = RES ? nsx : G.wx, pzw = RES ? cw : G.ld;
-  auto psx = [&](int t) -> float* {
-    if constexpr (RES) return sm + Y.psix + t * Y.psix_n - sx0;
-    else return P.psix[t] + (size_t)i0 * G.wx;
-  };
-  auto psz = [&](int t) -> float* {
-    if constexpr (RES) return sm + Y.psiz + t * Y.psiz_n - sz0 * cw;
-    else return P.psiz[t] + j0;
-  };
-  // cell arrays (RES): acoustic dt·κ dt·irx dt·irz; elastic λ λ+2μ dt·μ dt·irx dt·irz;
+  // ψ of x term t at (row r, strip column s): psx(t)[r·nsx + s]; of z term t
+  // at (strip row s, tile column c): psz(t)[s·cw + c]
+  auto psx = [&](int t) -> float* { return sm + Y.psix + t * Y.psix_n - sx0; };
+  auto psz = [&](int t) -> float* { return sm + Y.psiz + t * Y.psiz_n - sz0 * cw; };
+  // cell arrays: acoustic dt·κ dt·irx dt·irz; elastic λ λ+2μ dt·μ dt·irx dt·irz;
   // viscoacoustic K_R dt·irx dt·irz b_l ε r_l
-  const size_t fs = (size_t)(P.f[1] - P.f[0]);   // pitch of fields and coefficients
   // ------------------------------------------------------------------ load
   if (tid == 0) s_abort = 0;
 #pragma unroll 1
   for (int k = tid; k < NF * FN / 4; k += NT) st4(sm + Y.field + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
-  if (RES)
 #pragma unroll 1
-    for (int k = tid; k < (Y.psix - Y.cell) / 4; k += NT) st4(sm + Y.cell + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
+  for (int k = tid; k < (Y.psix - Y.cell) / 4; k += NT) st4(sm + Y.cell + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
   __syncthreads();
   const ptrdiff_t ld_delta = w.load ? w.load - P.f[0] : 0;
 #pragma unroll 1
@@ -546,50 +536,43 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     const size_t g = (size_t)(i0 + r) * G.ld + j0 + c4;
 #pragma unroll
     for (int f = 0; f < NF; ++f) st4(own + f * FN + r * W + c4, ld4(P.f[f] + ld_delta + g));
-    if constexpr (RES) {
-      const int o = r * cw + c4;
-      auto scaled = [&](int a, const float* src) {
-        const float4 v = ldg4(src + g);
-        st4(cells + a * CN + o, make_float4(fmul(G.dt, v.x), fmul(G.dt, v.y), fmul(G.dt, v.z), fmul(G.dt, v.w)));
-      };
-      if constexpr (EL) {
-        st4(cells + 0 * CN + o, ldg4(P.coef[CE_LAM] + g));
-        st4(cells + 1 * CN + o, ldg4(P.coef[CE_L2M] + g));
-        scaled(2, P.coef[CE_MUXZ]);
-        scaled(3, P.coef[CE_IRX]);
-        scaled(4, P.coef[CE_IRZ]);
-      } else if constexpr (VISCO) {
-        st4(cells + 0 * CN + o, ldg4(P.coef[CV_KR] + g));
-        scaled(1, P.coef[CV_IRX]);
-        scaled(2, P.coef[CV_IRZ]);
+    const int o = r * cw + c4;
+    auto scaled = [&](int a, const float* src) {
+      const float4 v = ldg4(src + g);
+      st4(cells + a * CN + o, make_float4(fmul(G.dt, v.x), fmul(G.dt, v.y), fmul(G.dt, v.z), fmul(G.dt, v.w)));
+    };
+    if constexpr (EL) {
+      st4(cells + 0 * CN + o, ldg4(P.coef[CE_LAM] + g));
+      st4(cells + 1 * CN + o, ldg4(P.coef[CE_L2M] + g));
+      scaled(2, P.coef[CE_MUXZ]);
+      scaled(3, P.coef[CE_IRX]);
+      scaled(4, P.coef[CE_IRZ]);
+    } else if constexpr (VISCO) {
+      st4(cells + 0 * CN + o, ldg4(P.coef[CV_KR] + g));
+      scaled(1, P.coef[CV_IRX]);
+      scaled(2, P.coef[CV_IRZ]);
 #pragma unroll 1
-        for (int l = 0; l < nL; ++l) st4(cells + (3 + l) * CN + o, ldg4(P.coef[CV_B0 + l] + g));
+      for (int l = 0; l < nL; ++l) st4(cells + (3 + l) * CN + o, ldg4(P.coef[CV_B0 + l] + g));
 #pragma unroll 1
-        for (int l = 0; l <= nL; ++l) st4(cells + (3 + nL + l) * CN + o, ld4(P.f[V_EPS + l] + ld_delta + g));
-        *reinterpret_cast<uchar4*>(qsm + o) = *reinterpret_cast<const uchar4*>(P.qidx + g);
-      } else {
-        scaled(0, P.coef[CA_KAPPA]);
-        scaled(1, P.coef[CA_IRX]);
-        scaled(2, P.coef[CA_IRZ]);
-      }
-    } else if (VISCO && ld_delta != 0) {
-#pragma unroll 1
-      for (int l = 0; l <= nL; ++l) st4(P.f[V_EPS + l] + g, ld4(P.f[V_EPS + l] + ld_delta + g));
+      for (int l = 0; l <= nL; ++l) st4(cells + (3 + nL + l) * CN + o, ld4(P.f[V_EPS + l] + ld_delta + g));
+      *reinterpret_cast<uchar4*>(qsm + o) = *reinterpret_cast<const uchar4*>(P.qidx + g);
+    } else {
+      scaled(0, P.coef[CA_KAPPA]);
+      scaled(1, P.coef[CA_IRX]);
+      scaled(2, P.coef[CA_IRZ]);
     }
   }
-  if (RES || ld_delta != 0) {
 #pragma unroll
-    for (int t = 0; t < NPSI; ++t) {
+  for (int t = 0; t < NPSI; ++t) {
 #pragma unroll 1
-      for (int k = tid; k < th * nsx; k += NT) {
-        const int r = k / nsx, s = k - r * nsx;
-        psx(t)[r * pxw + sx0 + s] = (P.psix[t] + ld_delta)[(size_t)(i0 + r) * G.wx + sx0 + s];
-      }
+    for (int k = tid; k < th * nsx; k += NT) {
+      const int r = k / nsx, s = k - r * nsx;
+      psx(t)[r * nsx + sx0 + s] = (P.psix[t] + ld_delta)[(size_t)(i0 + r) * G.wx + sx0 + s];
+    }
 #pragma unroll 1
-      for (int k = tid; k < nsz * gw; k += NT) {
-        const int s = k / gw, c4 = 4 * (k - s * gw);
-        st4(psz(t) + (sz0 + s) * pzw + c4, ld4(P.psiz[t] + ld_delta + (size_t)(sz0 + s) * G.ld + j0 + c4));
-      }
+    for (int k = tid; k < nsz * gw; k += NT) {
+      const int s = k / gw, c4 = 4 * (k - s * gw);
+      st4(psz(t) + (sz0 + s) * cw + c4, ld4(P.psiz[t] + ld_delta + (size_t)(sz0 + s) * G.ld + j0 + c4));
     }
   }
 #pragma unroll 1
@@ -728,7 +711,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   auto inject_cell = [&](int q) -> float* {
     const int ij = w.inj.ij[q], s = w.inj.slot[q], i = ij >> 16, j = ij & 0xffff;
     if (VISCO && s >= V_EPS)
-      return RES ? cells + (3 + nL) * CN + (i - i0) * cw + j - j0 : P.f[V_EPS] + (size_t)i * G.ld + j;
+      return cells + (3 + nL) * CN + (i - i0) * cw + j - j0;
     return own + s * FN + (i - i0) * W + j - j0;
   };
   float* inj_cell = nullptr;
@@ -897,48 +880,28 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
 #pragma unroll
       for (int f = 0; f < NF; ++f) st4(P.f[f] + delta + g, ld4(own + f * FN + r * W + c4));
       if constexpr (VISCO) {
-        if (RES || delta != 0)
 #pragma unroll 1
-          for (int l = 0; l <= nL; ++l)
-            st4(P.f[V_EPS + l] + delta + g,
-                RES ? ld4(cells + (3 + nL + l) * CN + r * cw + c4) : ld4(P.f[V_EPS + l] + g));
+        for (int l = 0; l <= nL; ++l)
+          st4(P.f[V_EPS + l] + delta + g, ld4(cells + (3 + nL + l) * CN + r * cw + c4));
       }
     }
-    if (RES || delta != 0) {
 #pragma unroll
-      for (int t = 0; t < NPSI; ++t) {
+    for (int t = 0; t < NPSI; ++t) {
 #pragma unroll 1
-        for (int k = tid; k < th * nsx; k += NT) {
-          const int r = k / nsx, s = k - r * nsx;
-          (P.psix[t] + delta)[(size_t)(i0 + r) * G.wx + sx0 + s] = psx(t)[r * pxw + sx0 + s];
-        }
+      for (int k = tid; k < th * nsx; k += NT) {
+        const int r = k / nsx, s = k - r * nsx;
+        (P.psix[t] + delta)[(size_t)(i0 + r) * G.wx + sx0 + s] = psx(t)[r * nsx + sx0 + s];
+      }
 #pragma unroll 1
-        for (int k = tid; k < nsz * gw; k += NT) {
-          const int s = k / gw, c4 = 4 * (k - s * gw);
-          st4(P.psiz[t] + delta + (size_t)(sz0 + s) * G.ld + j0 + c4, ld4(psz(t) + (sz0 + s) * pzw + c4));
-        }
+      for (int k = tid; k < nsz * gw; k += NT) {
+        const int s = k / gw, c4 = 4 * (k - s * gw);
+        st4(P.psiz[t] + delta + (size_t)(sz0 + s) * G.ld + j0 + c4, ld4(psz(t) + (sz0 + s) * cw + c4));
       }
     }
   };
 
-  // per-cell coefficients of the thread's cells: resident, or from global
-  // memory (dtc: times dt, premultiplied when resident)
-  auto raw = [&](int a, int slot, int r, int c0, float (&v)[C]) {
-    if constexpr (RES) {
-      ldv<C>(cells + a * CN + r * cw + c0, v);
-    } else {
-      const float* p = P.coef[slot] + (size_t)(i0 + r) * G.ld + j0 + c0;
-#pragma unroll
-      for (int c = 0; c < C; ++c) v[c] = __ldg(p + c);
-    }
-  };
-  auto dtc = [&](int a, int slot, int r, int c0, float (&v)[C]) {
-    raw(a, slot, r, c0, v);
-    if constexpr (!RES) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) v[c] = fmul(G.dt, v[c]);
-    }
-  };
+  // cell array `a` (per-cell coefficients) of the thread's cells
+  auto coef = [&](int a, int r, int c0, float (&v)[C]) { ldv<C>(cells + a * CN + r * cw + c0, v); };
   // CPML memories of the thread's cells (edge CTAs): N terms at once, all
   // loaded before any is stored; d[n][c] ← corrected derivative
   auto strips_x = [&](auto first, auto& d, int r, const float4 (&ct)[C]) {
@@ -948,27 +911,27 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     for (int n = 0; n < N; ++n)
 #pragma unroll
       for (int c = 0; c < C; ++c)
-        q[n][c] = wave_strip_of(ct[c]) >= 0 ? psx(first + n)[r * pxw + wave_strip_of(ct[c])] : 0.f;
+        q[n][c] = wave_strip_of(ct[c]) >= 0 ? psx(first + n)[r * nsx + wave_strip_of(ct[c])] : 0.f;
 #pragma unroll
     for (int n = 0; n < N; ++n)
 #pragma unroll
       for (int c = 0; c < C; ++c)
         if (wave_strip_of(ct[c]) >= 0) {
           (*d[n])[c] = cpml((*d[n])[c], q[n][c], ct[c].x, ct[c].y);
-          psx(first + n)[r * pxw + wave_strip_of(ct[c])] = q[n][c];
+          psx(first + n)[r * nsx + wave_strip_of(ct[c])] = q[n][c];
         }
   };
   auto strips_z = [&](auto first, auto& d, int c0, const float4& rt, const float4 (&ct)[C]) {
     constexpr int N = sizeof(d) / sizeof(d[0]);
     float q[N][C];
 #pragma unroll
-    for (int n = 0; n < N; ++n) ldv<C>(psz(first + n) + wave_strip_of(rt) * pzw + c0, q[n]);
+    for (int n = 0; n < N; ++n) ldv<C>(psz(first + n) + wave_strip_of(rt) * cw + c0, q[n]);
 #pragma unroll
     for (int n = 0; n < N; ++n) {
 #pragma unroll
       for (int c = 0; c < C; ++c)
         if (wave_flags_of(ct[c]) & WAVE_OK) (*d[n])[c] = cpml((*d[n])[c], q[n][c], rt.x, rt.y);
-      stv<C>(psz(first + n) + wave_strip_of(rt) * pzw + c0, q[n]);
+      stv<C>(psz(first + n) + wave_strip_of(rt) * cw + c0, q[n]);
     }
   };
 
@@ -1098,8 +1061,8 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
       float ox[C], oz[C], kx[C], kz[C];
       ldv<C>(pvx, ox);
       ldv<C>(pvz, oz);
-      dtc(EL ? 3 : 1, EL ? CE_IRX : CA_IRX, r, c0, kx);
-      dtc(EL ? 4 : 2, EL ? CE_IRZ : CA_IRZ, r, c0, kz);
+      coef(EL ? 3 : 1, r, c0, kx);
+      coef(EL ? 4 : 2, r, c0, kz);
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         if (EDGE && !(wave_flags_of(ct[c]) & WAVE_OK)) continue;
@@ -1161,7 +1124,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         float out[C], kk[C];
         ldv<C>(pp, out);
         if constexpr (!VISCO) {
-          dtc(0, CA_KAPPA, r, c0, kk);
+          coef(0, r, c0, kk);
 #pragma unroll
           for (int c = 0; c < C; ++c) {
             if (!live[c]) continue;
@@ -1170,24 +1133,22 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
           }
         } else {
           const int o = r * cw + c0;
-          const size_t g = (size_t)(i0 + r) * G.ld + j0 + c0;
-          float* const pe = RES ? cells + (3 + nL) * CN + o : P.f[V_EPS] + g;
-          float* const pr = RES ? cells + (4 + nL) * CN + o : P.f[V_R0] + g;
-          const float* const pb = RES ? cells + 3 * CN + o : P.coef[CV_B0] + g;
-          const size_t pitch = RES ? (size_t)CN : fs;
-          const unsigned char* const pq = RES ? qsm + o : P.qidx + g;
+          float* const pe = cells + (3 + nL) * CN + o;
+          float* const pr = cells + (4 + nL) * CN + o;
+          const float* const pb = cells + 3 * CN + o;
+          const unsigned char* const pq = qsm + o;
           float ev[C], rl[kRelaxUnroll][C], bl[kRelaxUnroll][C], tot[C];
           int q[C];
           ldv<C>(pe, ev);
-          raw(0, CV_KR, r, c0, kk);
+          coef(0, r, c0, kk);
           // every mechanism's memory and coefficient before any is stored
 #pragma unroll
           for (int c = 0; c < C; ++c) q[c] = pq[c] * nL;
 #pragma unroll
           for (int l = 0; l < kRelaxUnroll; ++l)
             if (l < nL) {
-              ldv<C>(pr + l * pitch, rl[l]);
-              ldv<C>(pb + l * pitch, bl[l]);
+              ldv<C>(pr + l * CN, rl[l]);
+              ldv<C>(pb + l * CN, bl[l]);
             }
           float inc[C];
 #pragma unroll
@@ -1204,7 +1165,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
                 if (live[c]) rl[l][c] = rv;
                 tot[c] = l == 0 ? rv : fadd(tot[c], rv);
               }
-              stv<C>(pr + l * pitch, rl[l]);
+              stv<C>(pr + l * CN, rl[l]);
             }
 #pragma unroll
           for (int c = 0; c < C; ++c) {
@@ -1252,9 +1213,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         ldv<C>(pxx, oxx);
         ldv<C>(pzz, ozz);
         ldv<C>(pxz, oxz);
-        raw(0, CE_LAM, r, c0, lam);
-        raw(1, CE_L2M, r, c0, l2m);
-        dtc(2, CE_MUXZ, r, c0, dmu);
+        coef(0, r, c0, lam);
+        coef(1, r, c0, l2m);
+        coef(2, r, c0, dmu);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (!live[c]) continue;
@@ -1305,10 +1266,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
         }
       } else if (!surface) {
         add(own + A_P * FN + src_o, amp);
-        if constexpr (VISCO) {
-          const size_t g = (size_t)G.src_iz * G.ld + G.src_ix;
-          add(RES ? cells + (3 + nL) * CN + src_e : P.f[V_EPS] + g, amp_eps);
-        }
+        if constexpr (VISCO) add(cells + (3 + nL) * CN + src_e, amp_eps);
       }
     }
     __syncthreads();
@@ -1372,10 +1330,9 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
             const int r = q / gw, c4 = 4 * (q - r * gw);
 #pragma unroll
             for (int f = 0; f < NF; ++f) scale4(own + f * FN + r * W + c4);
-            const size_t g = (size_t)(i0 + r) * G.ld + j0 + c4;
 #pragma unroll 1
             for (int l = 0; l <= nL; ++l)
-              scale4(RES ? cells + (3 + nL + l) * CN + r * cw + c4 : P.f[V_EPS + l] + g);
+              scale4(cells + (3 + nL + l) * CN + r * cw + c4);
           }
         }
       }
@@ -1400,7 +1357,6 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
 
 // Launch k_wave for an engine: `grid` CTAs (at most one per SM), `smem` bytes
 // of dynamic shared memory (wave.cu).
-cudaError_t wave_launch(int engine, int cells, bool res, const WaveSet& S, int grid, int smem, int smem_max,
-                        cudaStream_t st);
+cudaError_t wave_launch(int engine, int cells, const WaveSet& S, int grid, int smem, int smem_max, cudaStream_t st);
 
 }  // namespace ertm

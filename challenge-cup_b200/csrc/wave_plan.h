@@ -71,8 +71,8 @@ WAVE_HD inline int wave_r4(int n) { return (n + 3) / 4 * 4; }
 // pad: floats between the rows of a halo field beyond its own cells.  8 holds
 // the halo; with 32 the rows' first cells continue the bank sequence of the
 // cells before them, so a warp that spans rows has no bank conflicts.
-WAVE_HD inline WaveLayout wave_layout(bool elastic, bool visco, int L, bool res, int pad, int th, int gw,
-                                      int nsx, int nsz, int n_epi, int n_src, int n_acc) {
+WAVE_HD inline WaveLayout wave_layout(bool elastic, bool visco, int L, int pad, int th, int gw, int nsx,
+                                      int nsz, int n_epi, int n_src, int n_acc) {
   WaveLayout y;
   const int nf = elastic ? 5 : 3, nx = elastic ? 2 : 1, n_psi = elastic ? 4 : 2;
   y.cw = 4 * gw;
@@ -84,9 +84,9 @@ WAVE_HD inline WaveLayout wave_layout(bool elastic, bool visco, int L, bool res,
   o += nf * y.field_n;
   y.cell = o;
   y.cell_n = th * y.cw;
-  o += res ? (visco ? 4 + 2 * L : (elastic ? 5 : 3)) * y.cell_n : 0;
+  o += (visco ? 4 + 2 * L : (elastic ? 5 : 3)) * y.cell_n;
   y.qidx = o;
-  o += res && visco ? wave_r4(th * gw) : 0;   // one byte per cell
+  o += visco ? wave_r4(th * gw) : 0;   // one byte per cell
   y.epi = o;
   o += n_epi * y.cell_n;
   y.src = o;
@@ -94,10 +94,10 @@ WAVE_HD inline WaveLayout wave_layout(bool elastic, bool visco, int L, bool res,
   y.acc = o;
   o += 2 * n_acc * y.cell_n;
   y.psix = o;
-  y.psix_n = res ? wave_r4(th * nsx) : 0;
+  y.psix_n = wave_r4(th * nsx);
   o += n_psi * y.psix_n;
   y.psiz = o;
-  y.psiz_n = res ? nsz * y.cw : 0;
+  y.psiz_n = nsz * y.cw;
   o += n_psi * y.psiz_n;
   y.col = o;
   o += 4 * y.cw;
@@ -124,7 +124,6 @@ struct WavePlan {
   int cells = 1;      // neighbouring cells of a thread's block
   int thmax = 0, n_src = 0, n_acc = 0;
   std::vector<int16_t> cut;   // see wave_tile
-  bool res = false;
   int pad = 8;        // halo-field row padding (wave_layout)
   int smem = 0;       // bytes
   int64_t half = 0;   // exchange units per CTA and phase
@@ -146,8 +145,8 @@ inline int wave_smem(const WaveGrid& h, const WavePlan& p, const WaveNeeds& n) {
     int f, nsx, nsz;
     wave_strip(4 * t.g0, std::min(4 * (t.g0 + t.gw), h.nxp), h.nxp, h.npx_l, h.npx_r, f, nsx);
     wave_strip(t.i0, t.i0 + t.th, h.nzp, h.npz_t, h.npz_b, f, nsz);
-    const WaveLayout y = wave_layout(h.elastic, h.visco, h.L, p.res, p.pad, t.th,
-                                     t.gw, nsx, nsz, n.n_epi, p.n_src, p.n_acc);
+    const WaveLayout y = wave_layout(h.elastic, h.visco, h.L, p.pad, t.th, t.gw, nsx, nsz,
+                                     n.n_epi, p.n_src, p.n_acc);
     most = std::max(most, y.total * 4);
   }
   return most;
@@ -180,7 +179,8 @@ void wave_cuts(int n, int k, int least, F&& weight, int16_t* cut) {
 // thread (small grids, one pass of 512) 0.4.  Elastic 401×601 (µs a step):
 // 6.9 so, 7.9 with equal cuts, 11.6 the worst; acoustic 301×201 3.4 with one
 // cell a thread, 4.6 with two.  Imaging sums that do not fit in shared memory
-// cost about two round trips to L2 a step, coefficients that do not fit more.
+// cost about two round trips to L2 a step; a grid whose coefficients do not
+// fit has no split.
 inline WavePlan make_wave_plan(const WaveGrid& h, int ncta, const WaveNeeds& n) {
   WavePlan best;
   const int ng = (h.nxp + 3) / 4, nx = h.elastic ? 2 : 1;
@@ -217,24 +217,22 @@ inline WavePlan make_wave_plan(const WaveGrid& h, int ncta, const WaveNeeds& n) 
       most = std::max(most, t.th * t.gw * 4);
     }
     p.half = (int64_t)2 * nx * p.thmax + (int64_t)2 * nx * 4 * gw;
-    // the most that fits: resident coefficients first, then resident sums,
-    // then conflict-free rows
+    // the most that fits: resident sums first, then conflict-free rows
     bool fits = false;
-    for (int k = 0; k < 8 && !fits; ++k) {
+    for (int k = 0; k < 4 && !fits; ++k) {
       p.n_acc = (k & 2) == 0 ? n.n_acc : 0;
       p.n_src = p.n_acc ? n.n_src : 0;
       p.pad = (k & 1) == 0 ? 32 : 8;
-      p.res = k < 4;
       p.smem = wave_smem(h, p, n);
       fits = p.smem <= WAVE_SMEM_MAX;
     }
     if (!fits) continue;
     // relative cost of a step: SMs left idle, the shape, equal cuts (measured
-    // 14 % with two cells a thread), a second pass of a few cells, sums and
-    // coefficients that do not fit
+    // 14 % with two cells a thread), a second pass of a few cells, sums that
+    // do not fit
     const double c = (double)ncta / p.ctas() * (1.0 + 0.03 * std::fabs(px - ideal)) *
                      (single ? 1.0 + 0.05 * std::fabs(strip - 0.4) : 1.0 + 0.09 * (1.6 - strip)) *
-                     (single && most > WAVE_NT * cells ? 1.3 : 1.0) * (p.n_acc < n.n_acc ? 1.25 : 1.0) * (p.res ? 1.0 : 2.0);
+                     (single && most > WAVE_NT * cells ? 1.3 : 1.0) * (p.n_acc < n.n_acc ? 1.25 : 1.0);
     if (!best.ok() || c < cost) {
       best = p;
       cost = c;

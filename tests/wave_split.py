@@ -23,7 +23,7 @@ extern "C" int wave_split(const int* g, int ncta, const int* n, int* out, int16_
   const WaveGrid h{g[0] != 0, g[1] != 0, g[2], g[3], g[4], g[5], g[6], g[7], g[8]};
   const WavePlan p = make_wave_plan(h, ncta, {n[0], n[1], n[2]});
   if (!p.ok()) return 0;
-  const int vals[] = {p.px, p.pz, p.cells, p.res ? 1 : 0, p.n_acc, p.smem};
+  const int vals[] = {p.px, p.pz, p.cells, p.n_acc, p.smem};
   std::memcpy(out, vals, sizeof(vals));
   std::copy(p.cut.begin(), p.cut.end(), cut);
   const WaveKey k = wave_key(p);
@@ -52,7 +52,6 @@ class Split:
     px: int
     pz: int
     cells: int
-    resident: bool       # coefficients in shared memory
     sums: int            # imaging sums in shared memory
     smem: int
     rows: np.ndarray     # row cuts
@@ -73,7 +72,7 @@ def split(engine: str, nz: int, nx: int, *, npml: int = 20, boundary: str = "cpm
     grid = (C.c_int * 9)(engine == "elastic", engine == "viscoacoustic", mechanisms if engine == "viscoacoustic" else 0,
                          nzp, nxp, wx, wx, top, wz)
     rows, cols = (np.zeros(0, np.int32),) * 2 if points is None else (np.ascontiguousarray(p, np.int32) for p in points)
-    out, cut, key = (C.c_int * 6)(), (C.c_int16 * 512)(), (C.c_int16 * 512)()
+    out, cut, key = (C.c_int * 5)(), (C.c_int16 * 512)(), (C.c_int16 * 512)()
     first, order = np.zeros(257, np.int32), np.zeros(max(1, rows.size), np.int32)
     as_int = lambda a: a.ctypes.data_as(C.POINTER(C.c_int))
     k = _shim().wave_split(grid, ctas, (C.c_int * 3)(n_epi, n_src, n_acc), out, cut, key, int(rows.size), as_int(rows),
@@ -82,7 +81,7 @@ def split(engine: str, nz: int, nx: int, *, npml: int = 20, boundary: str = "cpm
         return None
     px, pz = out[0], out[1]
     cuts = np.array(cut[: px + pz + 2])
-    return Split(px, pz, out[2], bool(out[3]), out[4], out[5], cuts[: pz + 1], cuts[pz + 1:], tuple(key[:k]),
+    return Split(px, pz, out[2], out[3], out[4], cuts[: pz + 1], cuts[pz + 1:], tuple(key[:k]),
                  first[: px * pz + 1], order[: rows.size])
 
 
