@@ -1409,6 +1409,10 @@ void launch_epilogue(Prop& P, const Epilogue& E) {
   ++g_launches;
 }
 
+// Whether the multi-step launches of runs that the calling thread sets up lose
+// their edge values (ertm_set_wave_drop).
+thread_local bool t_wave_drop = false;
+
 // A shot's splits and its position in the multi-step schedule.
 struct WaveShot {
   WavePlan whole, alone;   // the forward pass; a replay on every SM
@@ -1434,6 +1438,7 @@ struct ShotRun {
   int n_src = 1;               // source image fields stored per replayed step (P and/or S)
   DevBuf wave_dev, rec, acc, ck, rbuf[2], running, peak;   // wave_dev: the wavelet
   std::vector<int64_t> ck_step;
+  bool drop = false;           // multi-step launches lose their edges (tests)
   InjectPlanHost* plan = nullptr;
   double* num[MAX_EPI_IMAGES] = {};
   double* ril[MAX_EPI_IMAGES] = {};
@@ -1470,6 +1475,7 @@ void prepare_run(ShotRun& R, Prop& F, Prop& B, const ertm_migrate_config& cfg, c
     }
   R.F = &F;
   R.B = &B;
+  R.drop = t_wave_drop;
   CK(cudaMemsetAsync(F.status.p, 0, sizeof(uint32_t), st));
   CK(cudaMemsetAsync(B.status.p, 0, sizeof(uint32_t), st));
   R.cfg = cfg;
@@ -1691,8 +1697,9 @@ struct WaveRunner {
   int grid = 0, smem = 0, engine = 0, cells = 1;   // shared by the works of a launch
   double bytes = 0.0;
   explicit WaveRunner(cudaStream_t s) : st(s) {}
-  void begin() {
+  void begin(bool drop) {
     S = WaveSet{};
+    S.drop = drop ? 1 : 0;
     grid = smem = 0;
     bytes = 0.0;
   }
@@ -1838,7 +1845,7 @@ bool forward_wave(Prop& P, int nt, const float* dwave, const SampleSet& S, const
   WaveRunner run(P.st);
   for (int t = 0; t < nt; t += chunk) {
     const int m = std::min(chunk, nt - t);
-    run.begin();
+    run.begin(t_wave_drop);
     WaveWork& w = run.add(P, p, m);
     w.t0 = t;
     w.wavelet = dwave;
@@ -1986,7 +1993,7 @@ void wave_advance(WaveRunner& run, ShotRun& R, int budget, cudaStream_t st) {
   double lp = 0.0;
   while (R.phase != 4 && budget > 0) {
     const int most = std::min(budget, kWaveMaxSteps);
-    run.begin();
+    run.begin(R.drop);
     if (R.phase == 0) {
       const int t = R.t_f, m = std::min(most, R.nt - t);
       WaveWork& w = run.add(F, W.whole, m);
@@ -2871,6 +2878,10 @@ int32_t ertm_set_wave(int32_t mode) {
   });
 }
 
+int32_t ertm_set_wave_drop(int32_t enable) {
+  return guarded([&] { t_wave_drop = enable != 0; });
+}
+
 int32_t ertm_set_tma(int32_t enable) {
   return guarded([&] { g_tma.store(enable ? 1 : 0); });
 }
@@ -3227,7 +3238,8 @@ int32_t ertm_forward(void* prop, int32_t nt, const float* amps, int32_t n_comp, 
     DevBuf dwave(amps ? (size_t)nt * 4 : 0, P.st);
     if (amps) upload(dwave.p, amps, (size_t)nt * 4, P.st);
     if (forward_wave(P, nt, amps ? dwave.as<float>() : nullptr, S, plans)) {
-      REQUIRE(!(read_status(P, P.st) & STATUS_STALLED), "a wait between the CTAs of a launch ran out");
+      if (read_status(P, P.st) & STATUS_STALLED)
+        throw Error(ERTM_ERR_STATE, "forward: a wait between the CTAs of a launch ran out; reset the propagator");
       if (sampling) CK(cudaMemcpyAsync(out, o.p, o.bytes, cudaMemcpyDefault, P.st));
       CK(cudaStreamSynchronize(P.st));
       return;

@@ -40,7 +40,8 @@
 // 63.3 → 13.7 ms, the PP/PS migration 50.7 → 24.5 ms.
 //
 // Every wait is bounded: when a wait runs out the CTA sets STATUS_STALLED and
-// leaves; its neighbours' waits then run out too.  Co-residency is the
+// leaves; its neighbours' waits then run out too, and later launches on the
+// propagator return at once until its status is cleared.  Co-residency is the
 // cooperative launch's guarantee.
 //
 // Arithmetic: expression for expression that of the tile kernels, so fields,
@@ -169,7 +170,7 @@ struct WaveWork {
 };
 
 struct WaveSet {
-  int32_t n, pad_;
+  int32_t n, drop;                   // works; drop: edges go unread (tests)
   uint64_t* xbuf;                    // exchange buffer: per CTA 2 phases × half units × 2 words, in two planes
   int64_t half;                      // units per CTA and phase
   int64_t plane;                     // words per plane
@@ -523,12 +524,13 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
   // cell arrays: acoustic dt·κ dt·irx dt·irz; elastic λ λ+2μ dt·μ dt·irx dt·irz;
   // viscoacoustic K_R dt·irx dt·irz b_l ε r_l
   // ------------------------------------------------------------------ load
-  if (tid == 0) s_abort = 0;
+  if (tid == 0) s_abort = (*static_cast<volatile uint32_t*>(P.status) & STATUS_STALLED) ? 1 : 0;
 #pragma unroll 1
   for (int k = tid; k < NF * FN / 4; k += NT) st4(sm + Y.field + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
 #pragma unroll 1
   for (int k = tid; k < (Y.psix - Y.cell) / 4; k += NT) st4(sm + Y.cell + 4 * k, make_float4(0.f, 0.f, 0.f, 0.f));
   __syncthreads();
+  if (s_abort) return;   // an earlier launch of the run stalled: nothing to go on from
   const ptrdiff_t ld_delta = w.load ? w.load - P.f[0] : 0;
 #pragma unroll 1
   for (int k = tid; k < th * gw; k += NT) {
@@ -597,7 +599,10 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
     for (int k = tid; k < 2 * nu; k += NT) {
       const WaveUnit q = wave_unit(EL, k / nu, k % nu, T, w.px, w.pz, w.thmax, W);
       const int64_t at = ((int64_t)blockIdx.x * 2 + k / nu) * S.half;
-      const int64_t from = ((int64_t)(w.cta0 + q.nb) * 2 + k / nu) * S.half;
+      // dropped edges: the CTA waits at its own word of the other phase, which
+      // never holds the number it waits for
+      const int64_t from = S.drop ? ((int64_t)blockIdx.x * 2 + 1 - k / nu) * S.half
+                                  : ((int64_t)(w.cta0 + q.nb) * 2 + k / nu) * S.half;
       tab[k] = make_int4(q.slot * FN + q.src, q.slot * FN + q.dst, (int)(at + q.put), q.nb < 0 ? -1 : (int)(from + q.get));
     }
   }

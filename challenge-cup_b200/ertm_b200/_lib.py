@@ -82,6 +82,7 @@ _SIGNATURES = {
     "ertm_set_march": (_I32, [_I32]),
     "ertm_set_march_stress": (_I32, [_I32]),
     "ertm_set_wave": (_I32, [_I32]),
+    "ertm_set_wave_drop": (_I32, [_I32]),
     "ertm_set_autotune": (_I32, [_I32]),
     "ertm_set_tma": (_I32, [_I32]),
     "ertm_stage_timeouts": (C.c_int64, []),
@@ -178,6 +179,7 @@ def last_error() -> str:
 
 ERR_NONFINITE = -4
 STATUS_NONFINITE = 1
+STATUS_STALLED = 2
 
 
 def check(rc: int, what: str) -> None:

@@ -345,7 +345,8 @@ class Propagator2D:
     @property
     def status(self) -> int:
         """Device status bits after the queued steps (no reference counterpart):
-        bit 0 set once a step wrote NaN or infinity into a wavefield."""
+        bit 0 set once a step wrote NaN or infinity into a wavefield, bit 1
+        once a wait inside a multi-step launch ran out."""
         out = C.c_uint32()
         _lib.check(_lib.lib().ertm_prop_status(self._handle, C.byref(out)), "status")
         return int(out.value)

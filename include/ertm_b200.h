@@ -164,6 +164,12 @@ int32_t ertm_set_march_stress(int32_t enable);
  * 2 wherever they fit.
  * Results are identical in every mode. */
 int32_t ertm_set_wave(int32_t mode);
+/* For tests of failure handling: multi-step launches of runs that the calling
+ * thread sets up lose the edge values their SMs exchange.  The waits for them
+ * run out after about a second and the run fails with ERTM_ERR_STATE, as it
+ * would if an SM's launch stopped; the propagators' wavefields are then
+ * undefined until they are reset or migrated with again. */
+int32_t ertm_set_wave_drop(int32_t enable);
 /* Online autotuning of batched ticks (default on): the first ticks of each
  * group shape (engine, order, works, size class) try tile heights 8/16/32,
  * split off/on and one or two lanes, timed with CUDA events; the fastest is
