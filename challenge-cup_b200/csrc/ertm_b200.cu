@@ -3355,7 +3355,8 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
       if (!batch_tick(ptrs, S.dtable.as<DevProp>(), S.st)) break;
       ++S.ticks;
     }
-    // shots whose wavefields became non-finite leave the session; the others run on
+    // shots whose wavefields became non-finite or whose launches stalled leave
+    // the session; the others run on
     const int n_tab = (int)S.table.size();
     if (n_tab > 0) {
       if (S.status.bytes < (size_t)n_tab * 4) S.status = DevBuf((size_t)n_tab * 4, S.st);
@@ -3366,9 +3367,7 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
       CK(cudaStreamSynchronize(S.st));
       for (size_t i = 0; i < S.runs.size();) {
         const ShotRun& R = *S.runs[i];
-        if ((flags[R.fi] | flags[R.bi]) & STATUS_STALLED)
-          throw Error(ERTM_ERR_STATE, "session: a wait between the CTAs of a launch ran out");
-        if (!((flags[R.fi] | flags[R.bi]) & STATUS_NONFINITE)) {
+        if (!((flags[R.fi] | flags[R.bi]) & (STATUS_NONFINITE | STATUS_STALLED))) {
           ++i;
           continue;
         }

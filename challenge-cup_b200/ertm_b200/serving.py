@@ -24,7 +24,8 @@ A job whose shot fails to prepare (bad input, a mode the engine cannot image)
 fails alone; its shots already on the device run out and are dropped.  So
 does a job one of whose shots writes NaN or infinity into a wavefield on the
 device (an overflowing or unstable run): the session takes that shot out at
-the next poll and the job's future raises NonFiniteWavefieldError.
+the next poll and the job's future raises NonFiniteWavefieldError.  A shot
+whose launches stalled fails its job likewise, with SolverError.
 """
 
 from __future__ import annotations
@@ -41,7 +42,7 @@ from typing import Any, Callable
 import numpy as np
 
 from . import _lib
-from .exceptions import ImagingError, NonFiniteWavefieldError
+from .exceptions import ImagingError, NonFiniteWavefieldError, SolverError
 from .imaging import RTMImager, ShotMigrator
 from .types import ImageResult
 
@@ -304,7 +305,7 @@ class RTMServer:
                     continue
                 _lib.check(L.ertm_session_advance(handle, self.ticks_per_poll, done, len(done), C.byref(n_done)),
                            "session advance")
-                # shots whose wavefields became non-finite left the session: their jobs fail, others run on
+                # shots that became non-finite or stalled left the session: their jobs fail, others run on
                 while True:
                     _lib.check(L.ertm_session_take_failed(handle, failed, len(failed), C.byref(n_failed)),
                                "session failed shots")
@@ -401,15 +402,23 @@ class RTMServer:
         self._maybe_finish(js)
 
     def _shot_failed(self, slot: _Slot) -> None:
-        """A shot whose wavefield became non-finite on the device: its job
-        fails (once its other running shots have left the session); the
-        propagator pair is dropped rather than reused."""
+        """A shot whose wavefield became non-finite on the device, or whose
+        launches stalled: its job fails (once its other running shots have
+        left the session); the propagator pair is dropped rather than reused."""
         js = slot.job
         js.active -= 1
         self.stats["shots_failed"] = self.stats.get("shots_failed", 0) + 1
-        self._job_failed(js, NonFiniteWavefieldError(
-            f"shot {slot.index} of job {js.job.name!r}: a wavefield became non-finite (NaN or infinity) on the "
-            f"device"))
+        shot = f"shot {slot.index} of job {js.job.name!r}"
+        try:
+            stalled = (slot.mig.prop.status | slot.mig.back.status) & _lib.STATUS_STALLED
+        except SolverError as exc:
+            self._job_failed(js, exc)
+            return
+        if stalled:
+            self._job_failed(js, SolverError(f"{shot}: a wait inside a multi-step launch ran out"))
+        else:
+            self._job_failed(js, NonFiniteWavefieldError(
+                f"{shot}: a wavefield became non-finite (NaN or infinity) on the device"))
 
     def _maybe_finish(self, js: _Job) -> None:
         if js.active or js.future.done():

@@ -35,6 +35,7 @@ extern "C" {
 #define ERTM_ERR_NONFINITE (-4)
 /* propagator status bits (ertm_prop_status) */
 #define ERTM_STATUS_NONFINITE 1u
+#define ERTM_STATUS_STALLED 2u    /* a wait inside a multi-step launch ran out */
 
 /* engines (propagation.py:986-1001) */
 #define ERTM_ENGINE_ACOUSTIC 0
@@ -212,8 +213,9 @@ int32_t ertm_prop_info_get(void* prop, ertm_prop_info* info);
 int32_t ertm_prop_reset(void* prop);
 /* Status word of a propagator (ERTM_STATUS_* bits), read after its queued
  * work: the stress phase sets ERTM_STATUS_NONFINITE when it writes NaN or
- * infinity.  No reference counterpart (the reference lets such a run finish
- * with a non-finite image); the checks follow the finite-value contracts of
+ * infinity, a multi-step launch ERTM_STATUS_STALLED when a wait runs out.  No
+ * reference counterpart (the reference lets such a run finish with a
+ * non-finite image); the checks follow the finite-value contracts of
  * types.py:106-122, 202-236 on the run's outputs. */
 int32_t ertm_prop_status(void* prop, uint32_t* status);
 /* Propagator2D.set_source (propagation.py:264-267): padded node and mechanism. */
@@ -287,10 +289,11 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
 int32_t ertm_session_active(void* session);
 int64_t ertm_session_ticks(void* session);
 int32_t ertm_session_destroy(void* session);
-/* Shots of a session whose wavefields became non-finite: each advance checks
- * every active shot's propagators and takes such shots out of the session
- * (their accumulators are not finished); this returns and forgets up to cap
- * of their tags.  The other shots keep running. */
+/* Shots of a session whose wavefields became non-finite or whose launches
+ * stalled (ertm_prop_status of their propagators tells which): each advance
+ * checks every active shot's propagators and takes such shots out of the
+ * session (their accumulators are not finished); this returns and forgets up
+ * to cap of their tags.  The other shots keep running. */
 int32_t ertm_session_take_failed(void* session, int64_t* tags, int32_t cap, int32_t* n);
 
 /* lowpass_wavenumber (numerics.py:424-442): out = Re(ifft2(fft2(in) · taper))

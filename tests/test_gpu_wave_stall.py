@@ -73,3 +73,31 @@ def test_stalled_migration_fails_and_the_next_is_as_ever(engine, boundary):
             batch.migrate_shots([shot], model)
     assert np.array_equal(_images(imager.migrate_modes(shot, model))[0], want[0])
     assert np.array_equal(_images(batch.migrate_shots([shot], model)[0])[0], want[0])
+
+
+def test_stalled_shot_fails_its_job_alone():
+    from ertm_b200 import _lib
+    from ertm_b200.exceptions import NonFiniteWavefieldError, SolverError
+    from ertm_b200.serving import RTMServer, ServeJob
+    jobs = []
+    for engine, boundary in (("acoustic", "free"), ("elastic", "free"), ("viscoacoustic", "cpml")):
+        model, shot = _shot((96, 140), engine, boundary)
+        jobs.append((_imager(engine, boundary, shot.dt), model, shot))
+    want = [_images(imager.migrate_modes(shot, model))[0] for imager, model, shot in jobs]
+
+    def drop_second(what, job, index):   # runs in the serving thread, before the shot joins the session
+        if what == "prepare":
+            _lib.lib().ertm_set_wave_drop(int(job == 1))
+
+    with RTMServer(fault_hook=drop_second, ticks_per_poll=16) as server:
+        futures = [server.submit(ServeJob(shots=[shot], model=model, imager=imager)) for imager, model, shot in jobs]
+        with pytest.raises(SolverError, match="ran out") as failed:
+            futures[1].result(timeout=120)
+        assert not isinstance(failed.value, NonFiniteWavefieldError)
+        for k in (0, 2):
+            assert np.array_equal(futures[k].result(timeout=120).images[0].image, want[k])
+        # the server goes on
+        again = server.submit(ServeJob(shots=[jobs[1][2]], model=jobs[1][1], imager=jobs[1][0]))
+        assert np.array_equal(again.result(timeout=120).images[0].image, want[1])
+    s = server.summary()
+    assert s["jobs_failed"] == 1 and s["shots_failed"] == 1 and s["jobs_done"] == 3
