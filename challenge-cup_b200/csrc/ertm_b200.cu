@@ -430,6 +430,7 @@ struct WaveInjectHost {
 struct InjectPlanHost {
   DevBuf cell_field, cell_index, start, src, wa, wb;
   int n_cells = 0;
+  int most = 0;                    // contributions to one cell
   std::vector<int32_t> h_field, h_index, h_start, h_src;   // host copies
   std::vector<double> h_wa, h_wb;
   std::map<WaveKey, WaveInjectHost> wave;                  // by wave_key
@@ -663,6 +664,7 @@ InjectPlanHost& inject_plan(Prop& P, const std::vector<int>& comps, int64_t nt) 
   put(ip->wa, wa.data(), wa.size() * 8);
   put(ip->wb, wb.data(), wb.size() * 8);
   CK(cudaStreamSynchronize(P.st));
+  for (size_t k = 0; k + 1 < start.size(); ++k) ip->most = std::max(ip->most, (int)(start[k + 1] - start[k]));
   ip->h_field = std::move(cf);
   ip->h_index = std::move(cidx);
   ip->h_start = std::move(start);
@@ -1793,21 +1795,37 @@ struct WaveSampleHost {
   DevBuf cta, slot, ij, out;
 };
 
+// Without tables when there are too many (wave_samples).
 WaveSampleHost wave_sample(const Prop& P, const std::vector<SamplePlanHost*>& comps, const WavePlan& p) {
   struct Entry { int slot, i, j, out; };
   std::vector<Entry> all;
   const int ld = P.h.ld;
-  for (size_t c = 0; c < comps.size(); ++c) {
-    const SamplePlanHost& sp = *comps[c];
-    if (sp.kind == SAMPLE_ZERO) continue;
-    for (int r = 0; r < sp.n; ++r) {
-      if (!sp.h_valid[r]) continue;
-      for (int corner = 0; corner < 4; ++corner)
-        all.push_back({sp.kind == SAMPLE_PRESSURE ? -1 : sp.slot, sp.h_cell[r] / ld + (corner >> 1),
-                       sp.h_cell[r] % ld + (corner & 1), 4 * ((int)c * sp.n + r) + corner});
+  const WaveGrid grid = wave_grid(P.h);
+  auto each = [&](auto&& f) {
+    for (size_t c = 0; c < comps.size(); ++c) {
+      const SamplePlanHost& sp = *comps[c];
+      if (sp.kind == SAMPLE_ZERO) continue;
+      for (int r = 0; r < sp.n; ++r) {
+        if (!sp.h_valid[r]) continue;
+        const int i = sp.h_cell[r] / ld, j = sp.h_cell[r] % ld;
+        for (int corner = 0; corner < 4; ++corner)
+          f(Entry{sp.kind == SAMPLE_PRESSURE ? -1 : sp.slot, i + (corner >> 1), j + (corner & 1),
+                  4 * ((int)c * sp.n + r) + corner});
+      }
     }
+  };
+  if (t_wave != 2) {   // counted before anything is built
+    const WaveOwner own(grid, p);
+    std::vector<int64_t> count(p.ctas(), 0);
+    int64_t corners = 0, most = 0;
+    each([&](const Entry& e) {
+      ++corners;
+      most = std::max(most, ++count[own.of(e.i, e.j)]);
+    });
+    if (!wave_samples(corners, most)) return {};
   }
-  const WaveGroups g = wave_groups(wave_grid(P.h), p, (int)all.size(),
+  each([&](const Entry& e) { all.push_back(e); });
+  const WaveGroups g = wave_groups(grid, p, (int)all.size(),
                                    [&](int k) { return std::make_pair(all[k].i, all[k].j); });
   std::vector<int32_t> slot, ij, out;
   for (const int32_t k : g.order) {
@@ -1831,13 +1849,16 @@ bool wave_wanted(const WavePlan& p) { return p.ok() && t_wave != 1; }
 // does not qualify.
 bool forward_wave(Prop& P, int nt, const float* dwave, const SampleSet& S, const std::vector<SamplePlanHost*>& comps) {
   const bool comp = P.h.engine == ENGINE_VISCO && P.cfg.compensation;
-  if (nt < 2 || comp) return false;
+  if ((t_wave == 2 ? nt < 2 : !wave_long(nt)) || comp) return false;
   const WavePlan p = wave_plan(P, sm_count(), {});
   if (!wave_wanted(p)) return false;
   const int n = S.count ? S.plan[0].n : 0;
   const int64_t stride = 4 * (int64_t)S.count * n;
   WaveSampleHost sh;
-  if (stride) sh = wave_sample(P, comps, p);
+  if (stride) {
+    sh = wave_sample(P, comps, p);
+    if (!sh.cta.p) return false;
+  }
   // corner values of one launch: at most 32 MB
   const int chunk = stride ? (int)std::max<int64_t>(16, std::min<int64_t>(kWaveMaxSteps, (int64_t(8) << 20) / stride))
                            : kWaveMaxSteps;
@@ -1877,6 +1898,7 @@ bool wave_shot(ShotRun& R) {
   const Prop& B = *R.B;
   if (R.fwd_unfused) return false;
   if (F.h.engine == ENGINE_VISCO && F.cfg.compensation) return false;
+  if (R.plan && !wave_injects(R.plan->most) && t_wave != 2) return false;
   const int n = sm_count();
   WaveNeeds nf, nb;
   if (F.h.engine == ENGINE_ELASTIC) {   // pressure engines image p where it is

@@ -261,6 +261,28 @@ inline bool wave_few(bool visco, int64_t cells, int together) {
   return cells <= 200000 && together <= (visco ? 2 : 3);
 }
 
+// Whether modelling `nt` steps takes multi-step launches: fewer than 8 cost
+// more to set up than they save (step by step and so, ms: 301×201 acoustic 2
+// steps 0.137 and 0.179, 5 steps 0.178 and 0.187, 8 steps 0.232 and 0.191;
+// 401×601 elastic 0.184 and 0.240, 0.240 and 0.269, 0.307 and 0.282).
+inline bool wave_long(int nt) { return nt >= 8; }
+
+// Whether `corners` receiver corner values a step, at most `most` of them in
+// one CTA, are few enough: the CTA writes its own, 512 at a time, while the
+// others wait, and the host groups all of them once per call.  200 steps, step
+// by step and so, ms: 16,000 receivers in a row on 301×201 acoustic (64,000
+// corners, 7,700 in a CTA) 5.2 and 3.7, two components of as many on 401×601
+// elastic (21,800 in a CTA) 7.6 and 8.6; 60,000 all over 301×201 (240,000
+// corners, 1,600 in a CTA) 14.9 and 15.3.
+inline bool wave_samples(int64_t corners, int64_t most) { return corners <= 131072 && most <= 8192; }
+
+// Whether an injection that adds at most `most` record values to one cell is
+// spread thin enough: a thread adds them one after the other between two
+// steps.  Migrations of 200 steps with receivers in a row, step by step and so,
+// ms: 401×601 elastic 20 values a cell 12.8 and 9.3, 80 values 15.6 and 20.1;
+// 801×601 acoustic 40 values 14.0 and 12.0, 150 values 19.0 and 36.1.
+inline bool wave_injects(int most) { return most <= 48; }
+
 // CTA of each padded cell's row and column group.
 struct WaveOwner {
   std::vector<int> tr, tc;

@@ -7,7 +7,7 @@ import itertools
 import numpy as np
 import pytest
 
-from wave_split import few_shots, split
+from wave_split import few_shots, split, takes
 
 # what a work keeps in shared memory beside the fields: (P/S fields, stored source fields, imaging sums)
 _NEEDS = {"acoustic": [(0, 0, 0), (0, 1, 1), (0, 1, 2), (0, 1, 3)],
@@ -54,3 +54,11 @@ def test_many_shots_share_ticks(engine):
     for nz, nx in ((256, 256), (330, 400)):
         assert all(few_shots(engine, nz, nx, n) for n in (1, 2))
         assert not any(few_shots(engine, nz, nx, n) for n in (4, 8, 45))
+
+
+def test_short_runs_and_dense_receivers_go_step_by_step():
+    """Calls that multi-step launches would slow down keep one launch pair per step."""
+    assert takes() and takes(8) and takes(corners=4 * 4 * 151, most=600, injected=12)
+    assert not any(takes(nt) for nt in (1, 2, 5))
+    assert not takes(corners=4 * 60000) and not takes(corners=100000, most=18000)
+    assert takes(injected=40) and not takes(injected=80)

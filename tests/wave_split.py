@@ -33,6 +33,9 @@ extern "C" int wave_split(const int* g, int ncta, const int* n, int* out, int16_
   std::copy(q.order.begin(), q.order.end(), order);
   return (int)k.size();
 }
+extern "C" int wave_takes(int nt, int64_t corners, int64_t most, int injected) {
+  return wave_long(nt) && wave_samples(corners, most) && wave_injects(injected);
+}
 extern "C" int wave_few_shots(int visco, int64_t cells, int together) { return wave_few(visco != 0, cells, together); }
 """
 
@@ -88,3 +91,9 @@ def split(engine: str, nz: int, nx: int, *, npml: int = 20, boundary: str = "cpm
 def few_shots(engine: str, nz: int, nx: int, together: int) -> bool:
     """Whether shots of a batch or session take multi-step launches."""
     return bool(_shim().wave_few_shots(int(engine == "viscoacoustic"), C.c_int64((nz + 10) * (nx + 10)), together))
+
+
+def takes(nt: int = 1000, *, corners: int = 0, most: int = 0, injected: int = 0) -> bool:
+    """Whether modelling or migration of so many steps, receiver corners and values injected into a cell takes
+    multi-step launches."""
+    return bool(_shim().wave_takes(nt, C.c_int64(corners), C.c_int64(most), injected))
