@@ -17,9 +17,11 @@ NT = 90
 
 
 def _shot(shape, engine, boundary):
-    from ertm_b200.types import ReceiverSpec, ShotRecord
+    from ertm_b200.types import ReceiverSpec, ShotRecord, SourceSpec
     model, src, rec, dt, nt, _ = _case(*shape, engine, NT, boundary)
     nz, nx = shape
+    # deep enough for the image to leave the absorbing strips
+    src = SourceSpec(x=src.x, z=10.0 * (nz // 2), f0=src.f0, delay=src.delay, mechanism=src.mechanism)
     # every column near the surface, and a well
     x = np.concatenate([rec.x, np.arange(nx) * 10.0, np.full(nz, 10.0 * (nx // 2))])
     z = np.concatenate([rec.z, np.full(nx, 20.0), np.arange(nz) * 10.0])
@@ -35,11 +37,13 @@ def _imager(engine, boundary, dt, condition="normalized"):
     from ertm_b200 import ImagingConfig, QConfig, RTMImager, SolverConfig
     q = QConfig(enabled=True, model="gsls", alpha_c=1.0, f_ref=20.0, f_max=40.0, amplitude_cap=50.0,
                 lowpass_interval=20, n_mechanisms=3) if engine == "viscoacoustic" else None
-    return RTMImager(ImagingConfig(mode="pp", condition=condition, separation="divcurl", checkpoint_mb=64.0),
+    return RTMImager(ImagingConfig(mode="pp", condition=condition, separation="divcurl", checkpoint_mb=64.0,
+                                     start_periods=0.0),
                      SolverConfig(nt=NT, dt=dt, order=8, boundary=boundary, engine=engine), q)
 
 
 def _images(results):
+    assert all(r.image.any() for r in results)
     return [r.image for r in results]
 
 
