@@ -11,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -40,24 +41,25 @@ def build(force: bool = False, ptxas_verbose: bool = False) -> Path:
     flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-O3"]
     if ptxas_verbose:
         flags.append("-Xptxas=-v")
-    objects = [OUT.parent / f"{src.stem}.o" for src in SOURCES]
-    # the translation units compile side by side
-    procs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(obj), str(src)], stdout=subprocess.PIPE,
-                              stderr=subprocess.STDOUT, text=True) for src, obj in zip(SOURCES, objects)]
-    logs = [p.communicate()[0] for p in procs]
-    tmp = OUT.with_suffix(".so.tmp")
-    link = [nvcc(), *ARCH, "-shared", "-o", str(tmp), *map(str, objects), "-lcufft"]
-    for p, log in zip(procs, logs):
-        if p.returncode != 0 or ptxas_verbose:
-            sys.stderr.write(log)
-    if any(p.returncode != 0 for p in procs):
-        raise RuntimeError("nvcc failed")
-    res = subprocess.run(link, capture_output=True, text=True)
+    # the translation units compile side by side; objects and the new library
+    # have names of their own, so builds do not meet and failures leave nothing
+    tmp = OUT.with_suffix(f".so.{os.getpid()}.tmp")
+    with tempfile.TemporaryDirectory(prefix="ertm-build-") as d:
+        objects = [Path(d) / f"{src.stem}.o" for src in SOURCES]
+        procs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(obj), str(src)], stdout=subprocess.PIPE,
+                                  stderr=subprocess.STDOUT, text=True) for src, obj in zip(SOURCES, objects)]
+        logs = [p.communicate()[0] for p in procs]
+        for p, log in zip(procs, logs):
+            if p.returncode != 0 or ptxas_verbose:
+                sys.stderr.write(log)
+        if any(p.returncode != 0 for p in procs):
+            raise RuntimeError("nvcc failed")
+        link = [nvcc(), *ARCH, "-shared", "-o", str(tmp), *map(str, objects), "-lcufft"]
+        res = subprocess.run(link, capture_output=True, text=True)
     if res.returncode != 0:
+        tmp.unlink(missing_ok=True)
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError(f"nvcc (link) failed with exit code {res.returncode}")
-    for obj in objects:
-        obj.unlink()
     os.replace(tmp, OUT)
     return OUT
 
