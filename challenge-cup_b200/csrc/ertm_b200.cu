@@ -2596,21 +2596,27 @@ bool batch_tick(std::vector<ShotRun*>& runs, const DevProp* dt, cudaStream_t st)
   return true;
 }
 
-// Whether a shot of a batch or session runs through multi-step launches, with
-// `together` shots of its engine in flight, itself included.
-bool wave_in_batch(ShotRun& R, int together) {
-  const DevProp& h = R.F->h;
-  if (t_wave == 0 && !wave_few(h.engine == ENGINE_VISCO, (int64_t)h.nzp * h.nxp, together)) return false;
+// The small shots of each engine among the runs of a batch or session.
+struct WaveCount {
+  int n[3] = {};
+  static bool small(const ShotRun& R) { return wave_small((int64_t)R.F->h.nzp * R.F->h.nxp); }
+  void add(const ShotRun& R) { n[R.F->h.engine] += small(R) ? 1 : 0; }
+};
+
+// Whether a shot of a batch or session runs through multi-step launches.
+bool wave_in_batch(ShotRun& R, const WaveCount& flight) {
+  const int engine = R.F->h.engine;
+  if (t_wave == 0 && !(WaveCount::small(R) && wave_few(engine == ENGINE_VISCO, flight.n[engine]))) return false;
   return wave_shot(R);
 }
 
 void migrate_batch(std::vector<ShotRun>& runs, cudaStream_t st) {
   std::vector<ShotRun*> ptrs;
   WaveRunner run(st);
-  int count[3] = {};   // shots per engine
-  for (ShotRun& R : runs) ++count[R.F->h.engine];
+  WaveCount count;
+  for (ShotRun& R : runs) count.add(R);
   for (ShotRun& R : runs) {
-    if (wave_in_batch(R, count[R.F->h.engine])) wave_advance(run, R, INT_MAX, st);
+    if (wave_in_batch(R, count)) wave_advance(run, R, INT_MAX, st);
     else ptrs.push_back(&R);
   }
   std::vector<DevProp> table;
@@ -3349,12 +3355,12 @@ int32_t ertm_session_advance(void* session, int32_t max_ticks, int64_t* done_tag
     *n_done = 0;
     // shots in ticks, and shots in multi-step launches (as many steps each); a
     // shot keeps the route it gets when it first advances
-    int count[3] = {};   // shots in flight per engine
-    for (auto& R : S.runs) ++count[R->F->h.engine];
+    WaveCount count;
+    for (auto& R : S.runs) count.add(*R);
     std::vector<ShotRun*> all, ptrs;
     for (auto& R : S.runs) {
       if (!R->routed) {
-        wave_in_batch(*R, count[R->F->h.engine]);
+        wave_in_batch(*R, count);
         R->routed = true;
       }
       all.push_back(R.get());

@@ -241,9 +241,9 @@ inline WavePlan make_wave_plan(const WaveGrid& h, int ncta, const WaveNeeds& n) 
   return best;
 }
 
-// Whether a shot of a batch or session runs through multi-step launches, one
-// shot after another, rather than in ticks that all shots share: `cells` of its
-// padded grid, `together` shots of its engine in flight.  A tick's launches
+// Shots of a batch or session run through multi-step launches, one shot after
+// another, when their padded grids are small and at most a few small ones of an
+// engine are in flight; else in ticks that all shots share.  A tick's launches
 // cost much the same for one small shot as for several, a multi-step launch
 // follows the shots.  Ticks over multi-step launches, times of 200 steps of
 // batches on 256×256 to 440×440 grids:
@@ -255,11 +255,14 @@ inline WavePlan make_wave_plan(const WaveGrid& h, int ncta, const WaveNeeds& n) 
 //
 // (a viscoacoustic tick's low-passes share their transforms' launches).  Above
 // 200,000 cells two shots of an engine come out between 0.94 and 1.5; those
-// keep the ticks.  45 shots in flight in the serving loop: 32.5 shots/s in
-// ticks, 28.6 in multi-step launches.
-inline bool wave_few(bool visco, int64_t cells, int together) {
-  return cells <= 200000 && together <= (visco ? 2 : 3);
-}
+// keep the ticks.  The serving loop with 45 shots of 256×256 to 1024×512 in
+// flight: 33.0 shots/s so, 32.7 all in ticks, 28.6 with every small shot in
+// multi-step launches; the same jobs arriving at 6, 9, 12 and 16 a second, 99 %
+// of the shots done within 0.29, 0.41, 0.57 and 0.61 s so, 0.34, 0.50, 0.57 s
+// (6, 9, 12) all in ticks, 0.28, 0.38, 0.54 and 0.65 s with every small shot in
+// multi-step launches.  Counting large shots too gave 0.45 s at 9 a second.
+inline bool wave_small(int64_t cells) { return cells <= 200000; }
+inline bool wave_few(bool visco, int together) { return together <= (visco ? 2 : 3); }
 
 // Whether modelling `nt` steps takes multi-step launches: fewer than 8 cost
 // more to set up than they save (step by step and so, ms: 301×201 acoustic 2

@@ -36,7 +36,9 @@ extern "C" int wave_split(const int* g, int ncta, const int* n, int* out, int16_
 extern "C" int wave_takes(int nt, int64_t corners, int64_t most, int injected) {
   return wave_long(nt) && wave_samples(corners, most) && wave_injects(injected);
 }
-extern "C" int wave_few_shots(int visco, int64_t cells, int together) { return wave_few(visco != 0, cells, together); }
+extern "C" int wave_few_shots(int visco, int64_t cells, int together) {
+  return wave_small(cells) && wave_few(visco != 0, together);
+}
 """
 
 
@@ -89,7 +91,7 @@ def split(engine: str, nz: int, nx: int, *, npml: int = 20, boundary: str = "cpm
 
 
 def few_shots(engine: str, nz: int, nx: int, together: int) -> bool:
-    """Whether shots of a batch or session take multi-step launches."""
+    """Whether small shots of a batch or session take multi-step launches, so many of their engine in flight."""
     return bool(_shim().wave_few_shots(int(engine == "viscoacoustic"), C.c_int64((nz + 10) * (nx + 10)), together))
 
 
