@@ -32,10 +32,11 @@
 // shared-memory bandwidth.  So an edge CTA runs the straight-line form where
 // it can, cuts weigh CPML strips, and imaging sums stay in shared memory for
 // the launch where they fit (1000 elastic steps of 401×601: 7.9 → 6.7 ms,
-// an 800-step PP/PS migration 27.1 → 24.5 ms).  512 threads (128 registers, no
-// spills) beat 640, 768 and 1024 (64 registers): 1500 acoustic steps of 301×201
-// with 151 receivers 4.6 ms against 5.2, 5.4 and 5.7 ms; 2 × 2 cells a thread
-// were no faster than 2 × 1.  Against two or three launches a step: that run
+// an 800-step PP/PS migration 27.1 → 24.5 ms).  512 threads (up to 128
+// registers; the viscoacoustic two-cell form spills 108 bytes, the others none)
+// beat 640, 768 and 1024 (64 registers): 1500 acoustic steps of 301×201 with
+// 151 receivers 4.6 ms against 5.2, 5.4 and 5.7 ms; 2 × 2 cells a thread were
+// no faster than 2 × 1.  Against two or three launches a step: that run
 // 24.9 → 4.6 ms, the elastic one 20.9 → 6.7 ms, a 1500-step acoustic migration
 // 63.3 → 13.7 ms, the PP/PS migration 50.7 → 24.5 ms.
 //
@@ -773,7 +774,7 @@ __global__ void __launch_bounds__(WAVE_NT, 1) k_wave(const __grid_constant__ Wav
       run = false;
     if (run && w.n_acc) cp_async_wait_all();   // each thread staged its own cells
     if (run && !w.n_acc && ekind == EPI_IMAGE && !w.epi.kahan) {
-      // two blocks of the thread at a time (four spill registers)
+      // two blocks of the thread at a time
       constexpr int U = 2;
       int r = row0, c0 = col0;
 #pragma unroll 1

@@ -4,9 +4,10 @@
 models, grids, engines and lengths — through ``ertm_migrate_batch``: all
 shots advance together in ticks that share one velocity and one stress
 launch per (engine, order) group, and inside each shot the replay of block
-b−1 overlaps the backward pass over block b.  Every propagator performs the
-same steps in the same order as the plain one-shot path, so each image equals
-the plain path's image bit for bit.
+b−1 overlaps the backward pass over block b.  When few small shots of an
+engine are in the call, those run one after another in multi-step launches
+instead.  Every propagator performs the same steps in the same order as the
+plain one-shot path, so each image equals the plain path's image bit for bit.
 
 Shots are grouped so that a group's device memory (two propagators, the
 checkpoints, two replay buffers and the accumulators per shot) stays within a

@@ -6,8 +6,9 @@ by ``stack_images`` (pipeline.py:133-161).  ``RTMServer`` runs jobs of mixed
 engine, grid and length on one device:
 
 * a host thread owns a batch session (``ertm_session_*``): every admitted shot
-  advances in the session's lockstep ticks, shots that arrive while others run
-  join between ticks, and finished shots leave, so work of different jobs
+  advances in the session's lockstep ticks (or, while few small shots of its
+  engine are in flight, in multi-step launches of its own), shots that arrive
+  while others run join between ticks, and finished shots leave, so work of different jobs
   overlaps on the device;
 * shots are admitted in arrival order while their device footprint (two
   propagators, checkpoints, replay buffers, accumulators, record) fits the

@@ -270,8 +270,10 @@ typedef struct ertm_batch_shot {
 /* Batched form of ertm_migrate (the pipeline's shot loop, pipeline.py:277-283):
  * all shots advance together in ticks that share one velocity and one stress
  * launch per (engine, order) group; within a shot the replay of block b−1
- * overlaps the backward pass over block b.  Shots may differ in grid, engine,
- * length and condition.  Results equal n_shots separate ertm_migrate calls. */
+ * overlaps the backward pass over block b.  A few small shots of an engine run
+ * one after another in multi-step launches instead, which is faster (see
+ * ertm_set_wave).  Shots may differ in grid, engine, length and condition.
+ * Results equal n_shots separate ertm_migrate calls. */
 int32_t ertm_migrate_batch(int32_t n_shots, const ertm_batch_shot* shots);
 
 /* Batch sessions: the tick loop of ertm_migrate_batch made resumable, for a
@@ -281,7 +283,8 @@ int32_t ertm_migrate_batch(int32_t n_shots, const ertm_batch_shot* shots);
  * checkpoints; the shot's num/illum/rillum outputs must stay valid until
  * ertm_session_advance reports its tag done.  ertm_session_advance runs at
  * most max_ticks ticks, stopping early after the tick in which a shot
- * finishes, then writes the finished shots' accumulators and returns up to cap
+ * finishes, and as many steps of each shot in multi-step launches (a shot's
+ * route is chosen when it first advances, by the shots in flight), then writes the finished shots' accumulators and returns up to cap
  * of their tags.  A shot's propagators belong to the session until then. */
 int32_t ertm_session_create(void** session);
 int32_t ertm_session_add(void* session, const ertm_batch_shot* shot, int64_t tag);
